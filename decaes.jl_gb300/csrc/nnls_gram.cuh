@@ -663,6 +663,7 @@ static __device__ __noinline__ NnlsResult gram_nnls(GramWS g, double *x, double 
     out.nsetp = k;
     out.mode = mode;
     out.rnorm = sqrt(fma(mu2, xx, res));
+    out.xx = xx;
     return out;
 }
 

@@ -321,6 +321,7 @@ struct NnlsResult {
     int nsetp;
     int mode;
     double rnorm;
+    double xx;  // ||x||^2 (set by the mixed method's solver only)
 };
 
 // Main + secondary loops of unsafe_nnls! (tikh = false) and of its Tikhonov
