@@ -1079,15 +1079,25 @@ static __device__ DK_OUTLINE void fa_suggest(Search &S, double &xo, double &uo) 
         uo = r.y;
         return;
     }
-    int I0 = S.sidx[0];
-    double pl = g[I0 - 1], ul = S.u[I0 - 1], dl = S.du[I0 - 1], p = pl, u = ul;
-    #pragma unroll 1
-    for (int i = 2; i <= S.npts; ++i) {
-        int I = S.sidx[i - 1];
-        double pc = g[I - 1], uc = S.u[I - 1], dc = S.du[I - 1], xx, uu;
-        hermite_minimize(pl, pc, ul, uc, dl, dc, xx, uu);
-        if (uu < u) { p = xx; u = uu; }
-        pl = pc; ul = uc; dl = dc;
+    // One spline interval per lane (each costs ~60 FP64 instructions, redundant
+    // on every lane if taken one by one); the reference's scan keeps the first
+    // smallest value, starting from the first point's.
+    const int lane = threadIdx.x & 31, I0 = S.sidx[0];
+    double p = g[I0 - 1], u = S.u[I0 - 1];
+    if (!isnan_bits(u)) {
+        #pragma unroll 1
+        for (int c = 1; c < S.npts; c += 32) {
+            double x = 0, v = CUDART_NAN;
+            if (c + lane < S.npts) {
+                const int Il = S.sidx[c + lane - 1] - 1, Ir = S.sidx[c + lane] - 1;
+                hermite_minimize(g[Il], g[Ir], S.u[Il], S.u[Ir], S.du[Il], S.du[Ir], x, v);
+            }
+            __syncwarp();
+            long long key = isnan_bits(v) ? LLONG_MAX : okey(v);
+            int i = lane;
+            warp_keymin(key, i);
+            if (key < okey(u)) { p = bcast(x, i); u = bcast(v, i); }
+        }
     }
     xo = p;
     uo = u;
