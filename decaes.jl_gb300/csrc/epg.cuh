@@ -10,7 +10,7 @@
 // not-yet-consumed old value in a register.  Every state a step reads is the
 // previous step's value in both forms, so the curves are the same bits.
 //
-// State storage is strided so a warp can keep one curve per lane in shared
+// State storage (S_: a pointer to T, or a view indexed like one) is strided so a warp can keep one curve per lane in shared
 // memory with lane-contiguous layout: F(k) = S[(k-1)*st], Fbar(k) =
 // S[(ETL+k-1)*st], Z(k) = S[(2*ETL+k-1)*st].
 #pragma once
@@ -146,8 +146,8 @@ DX_HD void flat_state(const FlatCoef<T> &q, T F, T Fb, T Z, T &oF, T &oFb, T &oZ
 
 // epg_decay_curve! for the constant-flip kernel: impulse response, then
 // dc[i] = |m0 * dc[i]|.  S holds 3*ETL strided values (st apart).
-template <class T, class O>
-DX_HD void epg_flat_inplace(int ETL, const FlatCoef<T> &q, T *S, int st, O *dc, int dst) {
+template <class T, class S_, class O>
+DX_HD void epg_flat_inplace(int ETL, const FlatCoef<T> &q, S_ S, int st, O *dc, int dst) {
 #define EF(k) S[((k)-1) * st]
 #define EFb(k) S[(ETL + (k)-1) * st]
 #define EZ(k) S[(2 * ETL + (k)-1) * st]
@@ -249,8 +249,8 @@ DX_HD VecCoef<float> to_f32(const VecCoef<double> &k) {
 
 // epg_decay_curve! for EPGOptions (DualVector_Split_Dynamic), in place.
 // S holds 3*ETL strided values: state k's (x,y,z) at S[(3(k-1)+c)*st].
-template <class T, class O>
-DX_HD void epg_vec_inplace(int ETL, const VecCoef<T> &q, T *S, int st, O *dc, int dst) {
+template <class T, class S_, class O>
+DX_HD void epg_vec_inplace(int ETL, const VecCoef<T> &q, S_ S, int st, O *dc, int dst) {
 #define SX(k, c) S[(3 * ((k)-1) + (c)) * st]
     const T z0 = zero_of(q.m0);
     T M0x = q.b1 * q.m0, M0z = ((-q.c1) * q.m0) / 2;

@@ -43,16 +43,16 @@ __device__ __forceinline__ int tri(int j) { return (j * (j + 1)) >> 1; }
 __device__ __forceinline__ int gidx(int i, int j) { return i <= j ? tri(j) + i : tri(i) + j; }
 
 struct GramWS {
-    double *G;     // packed upper triangle of the Gram matrix, n(n+1)/2
-    double *L;     // packed strictly-lower unit factor of H_PP = L D L'
-    double *f;     // A'b
-    double *y;     // L^{-1} f_P
-    double *dd;    // pivots D (during a factorization: the running diagonal)
-    double *dinv;  // 1 / D
-    double *xp;    // x on P (xp[r] = x[P[r]])
-    int *P;        // passive columns, 0-based, k entries
-    int *pos;      // pos[j] = index of column j in P, or -1
-    int *lastP;    // passive set left by the previous solve (warm start)
+    ShD G;     // packed upper triangle of the Gram matrix, n(n+1)/2
+    ShD L;     // packed strictly-lower unit factor of H_PP = L D L'
+    ShD f;     // A'b
+    ShD y;     // L^{-1} f_P
+    ShD dd;    // pivots D (during a factorization: the running diagonal)
+    ShD dinv;  // 1 / D
+    ShD xp;    // x on P (xp[r] = x[P[r]])
+    ShI P;        // passive columns, 0-based, k entries
+    ShI pos;      // pos[j] = index of column j in P, or -1
+    ShI lastP;    // passive set left by the previous solve (warm start)
     int lastk;
     double bb;     // b'b
 };
@@ -103,7 +103,7 @@ __device__ __forceinline__ double widen(float f) {
 }
 
 // b'b.
-static __device__ void gram_bb(GramWS &g, int m, const double *b) {
+static __device__ void gram_bb(GramWS &g, int m, const ShD b) {
     const int lane = threadIdx.x & 31;
     double part = 0.0;
     #pragma unroll 1
@@ -113,7 +113,7 @@ static __device__ void gram_bb(GramWS &g, int m, const double *b) {
 
 // f = A'b from a row-major (transposed, m x n) basis in global memory: lanes
 // over columns, coalesced over each row.
-static __device__ __noinline__ void gram_rhs_t(GramWS &g, const double *AT, int m, int n, const double *b) {
+static __device__ __noinline__ void gram_rhs_t(GramWS &g, const double *AT, int m, int n, const ShD b) {
     const int lane = threadIdx.x & 31;
     #pragma unroll 1
     for (int j = lane; j < n; j += 32) {
@@ -135,7 +135,7 @@ static __device__ __noinline__ void gram_rhs_t(GramWS &g, const double *AT, int 
 // (the tensor-core grid products of the voxel), times their scale to the
 // normalized decay.
 static __device__ __noinline__ void gram_rhs_f32(GramWS &g, const float *F, int n, double scale, int m,
-                                                 const double *b) {
+                                                 const ShD b) {
     const int lane = threadIdx.x & 31;
     #pragma unroll 1
     for (int j = lane; j < n; j += 32) {
@@ -151,11 +151,11 @@ static __device__ __noinline__ void gram_rhs_f32(GramWS &g, const float *F, int 
 // EPG curves themselves, so the products are exact in FP64 and G is the Gram
 // matrix of the basis to FP64 rounding.  Lanes over columns for f and over the
 // n(n+1)/2 upper-triangle entries for G.
-static __device__ __noinline__ void gram_build_f32(GramWS &g, const float *As, int lda, int m, int n, const double *b) {
+static __device__ __noinline__ void gram_build_f32(GramWS &g, const Sh<float> As, int lda, int m, int n, const ShD b) {
     const int lane = threadIdx.x & 31;
     #pragma unroll 1
     for (int j = lane; j < n; j += 32) {
-        const float *aj = As + j * lda;
+        const Sh<float> aj = As + j * lda;
         double s0 = 0.0, s1 = 0.0;
         int i = 0;
         #pragma unroll 1
@@ -174,7 +174,7 @@ static __device__ __noinline__ void gram_build_f32(GramWS &g, const float *As, i
         while (tri(j) > p) --j;
         while (tri(j + 1) <= p) ++j;
         const int i = p - tri(j);
-        const float *ai = As + i * lda, *aj = As + j * lda;
+        const Sh<float> ai = As + i * lda, aj = As + j * lda;
         double s0 = 0.0, s1 = 0.0;
         int r = 0;
         #pragma unroll 1
@@ -207,8 +207,8 @@ static __device__ __noinline__ bool gram_refactor(GramWS g, int k, double mu2) {
     const int lane = threadIdx.x & 31;
     const int r0 = lane, r1 = lane + 32;
     const int p0 = r0 < k ? g.P[r0] : 0, p1 = r1 < k ? g.P[r1] : 0;
-    double *L0 = g.L + tri(r0 - 1), *L1 = g.L + tri(r1 - 1);
-    double *cu = g.xp;  // unscaled pivot column of the current step
+    const ShD L0 = g.L + tri(r0 - 1), L1 = g.L + tri(r1 - 1);
+    const ShD cu = g.xp;  // unscaled pivot column of the current step
     // strictly lower triangle and diagonal of H_PP, one row per lane, and each
     // row's pivot threshold tol * H_rr
     double th0 = 0.0, th1 = 0.0;
@@ -257,7 +257,7 @@ static __device__ __noinline__ bool gram_refactor(GramWS g, int k, double mu2) {
             while (a * (a + 1) / 2 > q) --a;
             while ((a + 1) * (a + 2) / 2 <= q) ++a;
             const int r = j + 1 + a, c = j + 1 + (q - a * (a + 1) / 2);
-            double *e = c == r ? g.dd + r : g.L + tri(r - 1) + c;
+            const ShD e = c == r ? g.dd + r : g.L + tri(r - 1) + c;
             *e = fma(-cu[r], g.L[tri(c - 1) + j], *e);
         }
         __syncwarp();
@@ -276,7 +276,7 @@ static __device__ __noinline__ bool gram_refactor(GramWS g, int k, double mu2) {
 static __device__ __noinline__ bool gram_append(GramWS g, int k, int t, double mu2) {
     const int lane = threadIdx.x & 31;
     const int r0 = lane, r1 = lane + 32;
-    const double *L0 = g.L + tri(r0 - 1), *L1 = g.L + tri(r1 - 1);
+    const ShD L0 = g.L + tri(r0 - 1), L1 = g.L + tri(r1 - 1);
     double v0 = r0 < k ? g.G[gidx(g.P[r0], t)] : 0.0, v1 = r1 < k ? g.G[gidx(g.P[r1], t)] : 0.0;
     #pragma unroll 1
     for (int i = 0; i < k; ++i) {
@@ -294,7 +294,7 @@ static __device__ __noinline__ bool gram_append(GramWS g, int k, int t, double m
     if (!gt_nonneg_bits(delta, kGramDepTol * htt)) return false;
     const double yt = g.f[t] - ly;
     if (!pos_bits(yt)) return false;
-    double *Lk = g.L + tri(k - 1);
+    const ShD Lk = g.L + tri(k - 1);
     if (r0 < k) Lk[r0] = w0;
     if (r1 < k) Lk[r1] = w1;
     if (lane == 0) {
@@ -317,7 +317,7 @@ static __device__ __noinline__ double2 gram_back(const GramWS g, int k) {
     #pragma unroll 1
     for (int i = k - 1; i >= 0; --i) {
         const double zi = lane_pick(u0, u1, i);
-        const double *Li = g.L + tri(i - 1);
+        const ShD Li = g.L + tri(i - 1);
         if (r0 < i) u0 = fma(-Li[r0], zi, u0);
         if (r1 < i) u1 = fma(-Li[r1], zi, u1);
     }
@@ -339,13 +339,13 @@ static __device__ __noinline__ double2 gram_back(const GramWS g, int k) {
 // absolute 1e-15 * bound.  Writes the min(m,n) largest square roots in
 // descending order to gam (zeros for the unresolved ones).  Uses y, xp, dd and
 // dinv as scratch (free before the first solve) and W (tri(n) doubles).
-static __device__ __noinline__ void gram_svdvals(GramWS g, double *W, int m, int n, double *gam) {
+static __device__ __noinline__ void gram_svdvals(GramWS g, const ShD W, int m, int n, double *gam) {
     const int lane = threadIdx.x & 31;
     const int np = tri(n);
 #pragma unroll 1
     for (int q = lane; q < np; q += 32) W[q] = g.G[q];
     __syncwarp();
-    double *d = g.dd, *e = g.dinv, *u = g.y, *qv = g.xp;
+    const ShD d = g.dd, e = g.dinv, u = g.y, qv = g.xp;
     // 1. tridiagonalization (Householder from the left and right, column k)
 #pragma unroll 1
     for (int k = 0; k + 2 < n; ++k) {
@@ -419,7 +419,7 @@ static __device__ __noinline__ void gram_svdvals(GramWS g, double *W, int m, int
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) bnd = fmax(bnd, __shfl_xor_sync(FULL, bnd, o));
     __syncwarp();
-    const double *e2 = W;
+    const ShD e2 = W;
     const double tau = 1e-14 * bnd, atol = 1e-15 * bnd;
     // Sturm count: eigenvalues of the tridiagonal matrix below x
     auto count_below = [&](double x) {
@@ -474,7 +474,7 @@ static __device__ __noinline__ void gram_svdvals(GramWS g, double *W, int m, int
 // holds the solution, idx its passive columns (1-based, nsetp entries) and
 // rnorm^2 = ||A x - b||^2 + mu2 ||x||^2.  mode = 1 when max_iter was reached
 // (the reference's cap 3n).
-static __device__ __noinline__ NnlsResult gram_nnls(GramWS g, double *x, double *wv, int *idx, int n, double mu2,
+static __device__ __noinline__ NnlsResult gram_nnls(GramWS g, const ShD x, const ShD wv, const ShI idx, int n, double mu2,
                                              int max_iter, int *lastk_io) {
     const int lane = threadIdx.x & 31;
     const int r0 = lane, r1 = lane + 32;

@@ -91,18 +91,42 @@ __device__ __forceinline__ void wsum2(double a, double b, double &sa, double &sb
     sb = __shfl_sync(FULL, v, 16);
 }
 
+// The kernels' dynamic shared memory.
+extern __shared__ __align__(16) double dk_smem[];
+
+// A pointer into it, held as a byte offset.  The solvers are out of line, and
+// through a plain pointer argument the compiler no longer knows the address
+// space: every access becomes a generic load or store with a 64-bit address (a
+// window check, a longer latency and two address instructions instead of one).
+// Indexing dk_smem itself keeps them 32-bit shared-memory accesses:
+// 240x240x1 x 48 echoes, L-curve: mixed 72.1 -> 66.3 ms; 120x120x1 FP64 method
+// 136.7 -> 131.2 ms, and no register spills in either kernel.
+template <class T>
+struct Sh {
+    int off;
+    __device__ __forceinline__ T *ptr() const { return reinterpret_cast<T *>(reinterpret_cast<char *>(dk_smem) + off); }
+    __device__ __forceinline__ T &operator[](int i) const { return ptr()[i]; }
+    __device__ __forceinline__ T &operator*() const { return *ptr(); }
+    __device__ __forceinline__ Sh operator+(int i) const { return Sh{off + i * (int)sizeof(T)}; }
+    __device__ __forceinline__ Sh &operator+=(int i) { off += i * (int)sizeof(T); return *this; }
+    template <class U>
+    __device__ __forceinline__ Sh<U> as() const { return Sh<U>{off}; }
+};
+using ShD = Sh<double>;
+using ShI = Sh<int>;
+
 // Per-warp views of the NNLS workspace (shared memory).
 struct NnlsWS {
-    double *C;    // lda x n, physical columns
-    double *b;    // lda (right-hand side, transformed in place)
-    double *zz;   // lda
-    double *x;    // n, indexed by original column (0-based)
-    double *w;    // n, indexed by logical position (0-based)
-    int *idx;     // n, 1-based original column at each logical position
-    unsigned char *diag;  // n, indexed by original column
-    double *rdiag;        // n, RN(1/diagonal) of each physical column in set P
-    int *posof;           // n, 1-based logical position of each physical column (inverse of idx)
-    int *zl;              // n, scratch list of physical columns
+    ShD C;    // lda x n, physical columns
+    ShD b;    // lda (right-hand side, transformed in place)
+    ShD zz;   // lda
+    ShD x;    // n, indexed by original column (0-based)
+    ShD w;    // n, indexed by logical position (0-based)
+    ShI idx;  // n, 1-based original column at each logical position
+    Sh<unsigned char> diag;  // n, indexed by original column
+    ShD rdiag;               // n, RN(1/diagonal) of each physical column in set P
+    ShI posof;               // n, 1-based logical position of each physical column (inverse of idx)
+    ShI zl;                  // n, scratch list of physical columns
     int lda;
 };
 
@@ -138,7 +162,7 @@ __device__ __forceinline__ double mdiv(double a, double b, double r) {
 
 __device__ __forceinline__ double &Aat(const NnlsWS &s, int i1, int j1) {
     // 1-based row i1 of logical column j1
-    return s.C[(i1 - 1) + (size_t)(s.idx[j1 - 1] - 1) * s.lda];
+    return s.C[(i1 - 1) + (s.idx[j1 - 1] - 1) * s.lda];
 }
 
 // Base.hypot for Float64 (C. F. Borges, "An Improved Algorithm for
@@ -167,7 +191,7 @@ static __device__ double jl_hypot(double x, double y) {
 static __device__ double warp_cah(const NnlsWS &s, int ip, int jp, int m) {
     const int lane = threadIdx.x & 31;
     if (ip > m) return 0.0;
-    double *col = s.C + (size_t)(s.idx[jp - 1] - 1) * s.lda;  // pivot column (0-based rows)
+    const ShD col = s.C + (s.idx[jp - 1] - 1) * s.lda;  // pivot column (0-based rows)
     double alpha = col[ip - 1];
     double part = 0.0;
     for (int i = ip + lane; i <= m; i += 32) part = fma(col[i - 1], col[i - 1], part);
@@ -224,13 +248,13 @@ static __device__ double warp_cah(const NnlsWS &s, int ip, int jp, int m) {
 static __device__ void warp_ahd(const NnlsWS &s, int n, double tau, int j1, int m1) {
     const int lane = threadIdx.x & 31;
     if (j1 >= m1) return;
-    const double *u = s.C + (size_t)(s.idx[j1 - 1] - 1) * s.lda;  // u[j1-1] is the diagonal; treated as 1
+    const ShD u = s.C + (s.idx[j1 - 1] - 1) * s.lda;  // u[j1-1] is the diagonal; treated as 1
     const int nz = warp_active_cols(s, n, j1 + 1);
     for (int r0 = 0; r0 < nz; r0 += 32) {
         int r = r0 + lane;
         if (r < nz) {
             const int p = s.zl[r];
-            double *a = s.C + (size_t)p * s.lda;
+            const ShD a = s.C + p * s.lda;
             double sm = fma(a[j1 - 1], 1.0, 0.0);
             for (int i = j1 + 1; i <= m1; ++i) sm = fma(a[i - 1], u[i - 1], sm);
             sm *= -tau;
@@ -255,7 +279,7 @@ static __device__ void warp_compute_dual(const NnlsWS &s, int n, int j1, int m1)
         int r = r0 + lane;
         if (r < nz) {
             const int p = s.zl[r];
-            const double *a = s.C + (size_t)p * s.lda;
+            const ShD a = s.C + p * s.lda;
             double sm = 0.0;
             for (int i = j1; i <= m1; ++i) sm = fma(a[i - 1], s.b[i - 1], sm);
             s.w[s.posof[p] - 1] = sm;
@@ -272,7 +296,7 @@ static __device__ void warp_solve_tri(const NnlsWS &s, int n) {
     __syncwarp();
     for (int j = n; j >= 1; --j) {
         const int pj = s.idx[j - 1] - 1;
-        const double *a = s.C + (size_t)pj * s.lda;
+        const ShD a = s.C + pj * s.lda;
         double zi = -mdiv(s.zz[j - 1], a[j - 1], s.rdiag[pj]);
         for (int i = 1 + lane; i <= j - 1; i += 32) s.zz[i - 1] = fma(a[i - 1], zi, s.zz[i - 1]);
         __syncwarp();
@@ -282,10 +306,10 @@ static __device__ void warp_solve_tri(const NnlsWS &s, int n) {
 }
 
 // Transposed solve (U' z = x) on the first n logical columns, src/NNLS.jl:524-537.
-static __device__ void warp_solve_tri_t(const NnlsWS &s, double *z, int n) {
+static __device__ void warp_solve_tri_t(const NnlsWS &s, ShD z, int n) {
     const int lane = threadIdx.x & 31;
     for (int j = 1; j <= n; ++j) {
-        const double *a = s.C + (size_t)(s.idx[j - 1] - 1) * s.lda;
+        const ShD a = s.C + (s.idx[j - 1] - 1) * s.lda;
         double part = 0.0;
         for (int l = 1 + lane; l <= j - 1; l += 32) part = fma(-a[l - 1], z[l - 1], part);
         double z1 = z[j - 1] + wsum(part);
@@ -370,7 +394,7 @@ static __device__ NnlsResult warp_nnls(const NnlsWS &s, int M, int n, int m0, bo
         __syncwarp();
         if (nsetp < n) warp_ahd(s, n, tau, nsetp, m);
         {
-            double *pc = s.C + (size_t)(s.idx[nsetp - 1] - 1) * s.lda;
+            const ShD pc = s.C + (s.idx[nsetp - 1] - 1) * s.lda;
             for (int i = nsetp + 1 + lane; i <= m; i += 32) pc[i - 1] = 0.0;
         }
         __syncwarp();
@@ -419,7 +443,7 @@ static __device__ NnlsResult warp_nnls(const NnlsWS &s, int M, int n, int m0, bo
                 __syncwarp();
                 if (imv != nsetp) {
                     for (int i = imv + 1; i <= nsetp; ++i) {
-                        double *ci = s.C + (size_t)(s.idx[i - 1] - 1) * s.lda;
+                        const ShD ci = s.C + (s.idx[i - 1] - 1) * s.lda;
                         double a = ci[i - 2], bb = ci[i - 1];
                         double sg = jl_hypot(a, bb);
                         double cc = a / sg, ss = bb / sg;
@@ -427,7 +451,7 @@ static __device__ NnlsResult warp_nnls(const NnlsWS &s, int M, int n, int m0, bo
                         const int pi = s.idx[i - 1] - 1;
                         for (int pj = lane; pj < n; pj += 32) {
                             if (pj == pi) continue;
-                            double *cj = s.C + (size_t)pj * s.lda;
+                            const ShD cj = s.C + pj * s.lda;
                             double p = cj[i - 2], r = cj[i - 1];
                             cj[i - 2] = fma(cc, p, __dmul_rn(ss, r));
                             cj[i - 1] = fma(-ss, p, __dmul_rn(cc, r));
@@ -496,14 +520,14 @@ static __device__ NnlsResult warp_nnls(const NnlsWS &s, int M, int n, int m0, bo
 // `data` is the (shared-memory) right-hand side; it is not modified.
 // Not inlined: every caller shares one copy of the NNLS code (instruction
 // cache), and the workspace views travel in registers.
-static __device__ __noinline__ NnlsResult warp_lsq(const NnlsWS s, const double *A, int m, int n, const double *data,
+static __device__ __noinline__ NnlsResult warp_lsq(const NnlsWS s, const double *A, int m, int n, const ShD data,
                                             bool tikh, double mu) {
     const int lane = threadIdx.x & 31;
     const int M = tikh ? m + n : m;
     // C[:, j] = A[:, j] (coalesced), padded rows zeroed
     for (int j = 0; j < n; ++j) {
         const double *aj = A + (size_t)j * m;
-        double *cj = s.C + (size_t)j * s.lda;
+        const ShD cj = s.C + j * s.lda;
         for (int i = lane; i < M; i += 32) cj[i] = (i < m) ? aj[i] : 0.0;
     }
     for (int i = lane; i < M; i += 32) s.b[i] = (i < m) ? data[i] : 0.0;
@@ -514,7 +538,7 @@ static __device__ __noinline__ NnlsResult warp_lsq(const NnlsWS s, const double 
         s.diag[j] = 0;
     }
     __syncwarp();
-    const double *an = s.C + (size_t)(n - 1) * s.lda;
+    const ShD an = s.C + (n - 1) * s.lda;
     double part = 0.0;
     for (int i = lane; i < m; i += 32) part = __dadd_rn(part, __dmul_rn(an[i], an[i]));
     double den = wsum(part);
@@ -529,7 +553,7 @@ static __device__ __noinline__ NnlsResult warp_lsq(const NnlsWS s, const double 
     for (int jb = 0; jb < n - 1; jb += 32) {
         int j = jb + lane;
         if (j < n - 1) {
-            const double *cj = s.C + (size_t)j * s.lda;
+            const ShD cj = s.C + j * s.lda;
             double wj = 0.0;
             for (int i = 0; i < m; ++i) wj = __dadd_rn(wj, __dmul_rn(cj[i], s.zz[i]));
             s.w[j] = wj;

@@ -49,8 +49,8 @@ constexpr bool kTcProducts = DECAES_TC_PRODUCTS != 0;
 struct Warp {
     const Params *P;
     NnlsWS s;
-    double *data;  // normalized decay data (shared), m
-    double *xout;  // saved solution (shared), n
+    ShD data;      // normalized decay data (shared), m
+    ShD xout;      // saved solution (shared), n
     double *A;     // per-voxel basis (global scratch), m x n
     double *scr;   // per-warp global scratch base
     double *sol_key, *sol_x;  // stored Tikhonov solutions: log mu keys, kSolCap x n
@@ -59,7 +59,7 @@ struct Warp {
     unsigned nnls_caps, loop_caps;
     // mixed method: normal-equation workspace and the staged basis (shared)
     GramWS g;
-    float *As32;   // FP32 basis staged in shared memory, column-major, leading dimension ldA
+    Sh<float> As32;  // FP32 basis staged in shared memory, column-major, leading dimension ldA
     int ldA;
     bool mixed;    // the mixed method (Params::mixed)
 };
@@ -719,16 +719,16 @@ static __device__ void warp_svdvals(Warp &w, double *gam) {
     const int m = P.m, n = P.n, lane = w.lane;
     const int r = m >= n ? m : n, c = m >= n ? n : m;
     const int ld = r | 1;
-    double *U = w.s.C;  // r x c, ld, fits in the lda x n workspace
+    const ShD U = w.s.C;  // r x c, ld, fits in the lda x n workspace
     #pragma unroll 1
     for (int j = 0; j < c; ++j)
         #pragma unroll 1
-        for (int i = lane; i < r; i += 32) U[i + (long)j * ld] = (m >= n) ? w.A[i + (long)j * m] : w.A[j + (long)i * m];
+        for (int i = lane; i < r; i += 32) U[i + j * ld] = (m >= n) ? w.A[i + (long)j * m] : w.A[j + (long)i * m];
     __syncwarp();
-    double *dv = w.s.zz, *ev = w.s.b;  // bidiagonal: c diagonal, c-1 superdiagonal entries
+    const ShD dv = w.s.zz, ev = w.s.b;  // bidiagonal: c diagonal, c-1 superdiagonal entries
     #pragma unroll 1
     for (int k = 0; k < c; ++k) {
-        const double *uk = U + (long)k * ld;
+        const ShD uk = U + k * ld;
         // left reflector H = I - tau v v', v = (x0 - alpha, x_{k+1..r-1}), on column k
         double ss = 0.0;
         #pragma unroll 1
@@ -745,7 +745,7 @@ static __device__ void warp_svdvals(Warp &w, double *gam) {
         if (tau != 0.0) {
             #pragma unroll 1
             for (int j = k + 1 + lane; j < c; j += 32) {
-                double *uj = U + (long)j * ld;
+                const ShD uj = U + j * ld;
                 double sdot = v0 * uj[k];
                 #pragma unroll 1
                 for (int i = k + 1; i < r; ++i) sdot = fma(uk[i], uj[i], sdot);
@@ -760,8 +760,8 @@ static __device__ void warp_svdvals(Warp &w, double *gam) {
             // right reflector on row k, columns k+1..c-1
             double sr = 0.0;
             #pragma unroll 1
-            for (int j = k + 2; j < c; ++j) { const double y = U[k + (long)j * ld]; sr = fma(y, y, sr); }
-            const double y0 = U[k + (long)(k + 1) * ld];
+            for (int j = k + 2; j < c; ++j) { const double y = U[k + j * ld]; sr = fma(y, y, sr); }
+            const double y0 = U[k + (k + 1) * ld];
             double beta = y0, w0 = 0.0, tau2 = 0.0;
             if (sr != 0.0) {
                 const double nrm = sqrt(fma(y0, y0, sr));
@@ -773,25 +773,25 @@ static __device__ void warp_svdvals(Warp &w, double *gam) {
             if (tau2 != 0.0) {
                 #pragma unroll 1
                 for (int i = k + 1 + lane; i < r; i += 32) {
-                    double sdot = w0 * U[i + (long)(k + 1) * ld];
+                    double sdot = w0 * U[i + (k + 1) * ld];
                     #pragma unroll 1
-                    for (int j = k + 2; j < c; ++j) sdot = fma(U[k + (long)j * ld], U[i + (long)j * ld], sdot);
+                    for (int j = k + 2; j < c; ++j) sdot = fma(U[k + j * ld], U[i + j * ld], sdot);
                     const double f = tau2 * sdot;
-                    U[i + (long)(k + 1) * ld] = fma(-f, w0, U[i + (long)(k + 1) * ld]);
+                    U[i + (k + 1) * ld] = fma(-f, w0, U[i + (k + 1) * ld]);
                     #pragma unroll 1
-                    for (int j = k + 2; j < c; ++j) U[i + (long)j * ld] = fma(-f, U[k + (long)j * ld], U[i + (long)j * ld]);
+                    for (int j = k + 2; j < c; ++j) U[i + j * ld] = fma(-f, U[k + j * ld], U[i + j * ld]);
                 }
             }
             __syncwarp();
         } else if (k + 1 < c) {
-            if (lane == 0) ev[k] = U[k + (long)(k + 1) * ld];
+            if (lane == 0) ev[k] = U[k + (k + 1) * ld];
             __syncwarp();
         }
     }
     // Golub-Kahan tridiagonal: squared off-diagonals o2 (2c-1, in U's storage)
     // and the Gershgorin bound
     const int N = 2 * c;
-    double *o2 = U;
+    const ShD o2 = U;
     double bnd = 0.0;
     #pragma unroll 1
     for (int j = lane; j < N; j += 32) {
@@ -1163,12 +1163,12 @@ static __device__ double flip_angle_search(Warp &w, double mx, long slot) {
 static __device__ void warp_basis(Warp &w, double alpha, double *out /* m x n, global */) {
     const Params &P = *w.P;
     const int m = P.m, n = P.n, lanes = P.epg_lanes, lane = w.lane;
-    double *S = w.s.C;  // 3*m*lanes doubles, lane-contiguous, over the C, b and zz regions
+    const ShD S = w.s.C;  // 3*m*lanes doubles, lane-contiguous, over the C, b and zz regions
     #pragma unroll 1
     for (int j0 = 0; j0 < n; j0 += lanes) {
         int j = j0 + lane;
         if (lane < lanes && j < n) {
-            double *Sl = S + lane;
+            const ShD Sl = S + lane;
             if (P.beta180) {
                 dx::FlatCoef<double> q = dx::flat_coef(alpha, P.TE, P.t2[j], P.T1);
                 dx::epg_flat_inplace(m, q, Sl, lanes, out + (long)j * m, 1);
@@ -1192,13 +1192,13 @@ static __device__ void warp_basis(Warp &w, double alpha, double *out /* m x n, g
 static __device__ void warp_basis_f32(Warp &w, double alpha) {
     const Params &P = *w.P;
     const int m = P.m, n = P.n, lanes = P.epg_lanes_f32, lane = w.lane;
-    float *S = reinterpret_cast<float *>(w.g.G);  // 3*m*lanes floats, lane-contiguous
+    const Sh<float> S = w.g.G.as<float>();  // 3*m*lanes floats, lane-contiguous
     float *Af = reinterpret_cast<float *>(w.scr + warp_scratch_f32_offset(m, n, P.K));
     #pragma unroll 1
     for (int j0 = 0; j0 < n; j0 += lanes) {
         int j = j0 + lane;
         if (lane < lanes && j < n) {
-            float *Sl = S + lane;
+            const Sh<float> Sl = S + lane;
             if (P.beta180) {
                 dx::FlatCoef<float> q = dx::to_f32(dx::flat_coef(alpha, P.TE, P.t2[j], P.T1));
                 dx::epg_flat_inplace(m, q, Sl, lanes, Af + (long)j * m, 1);
@@ -1364,7 +1364,7 @@ static __device__ void process_voxel(Warp &w, long v, long slot = 0) {
         // Each window sum runs in T2partSEcorr's loop order in a lane of its
         // own (total, SPWin, MPWin, sigmoid weights), so the fused maps equal
         // the standalone T2part of the saved distribution bit for bit.
-        const double *dv = w.s.w;
+        const ShD dv = w.s.w;
         bool anynan = false;
         #pragma unroll 1
         for (int j = lane; j < n; j += 32) anynan |= isnan(dv[j]);

@@ -11,7 +11,7 @@ namespace dk {
 
 // Points one warp's views at its shared-memory workspace p and global scratch
 // scr for the problem shape of P.
-static __device__ void warp_setup(Warp &w, const Params &P, double *p, double *scr) {
+static __device__ void warp_setup(Warp &w, const Params &P, ShD p, double *scr) {
     w.P = &P;
     w.mixed = P.mixed != 0;
     const int n = P.n, lda = P.lda;
@@ -22,28 +22,28 @@ static __device__ void warp_setup(Warp &w, const Params &P, double *p, double *s
         w.s.x = p; p += n;
         w.s.w = p; p += n;
         w.xout = p; p += n;
-        w.g.G = p; p += mixed_r1_doubles(m, n);
-        w.g.L = p; p += mixed_r2_doubles(m, n, P.reg == 2);
+        w.g.G = p; p += (int)mixed_r1_doubles(m, n);
+        w.g.L = p; p += (int)mixed_r2_doubles(m, n, P.reg == 2);
         w.g.f = p; p += n;
         w.g.y = p; p += n;
         w.g.dd = p; p += n;
         w.g.dinv = p; p += n;
         w.g.xp = p; p += n;
         p += 8;
-        int *ip = reinterpret_cast<int *>(p);
+        const ShI ip = p.as<int>();
         w.s.idx = ip;
         w.g.P = ip + n;
         w.g.pos = ip + 2 * n;
         w.g.lastP = ip + 3 * n;
         w.g.lastk = 0;
-        w.As32 = reinterpret_cast<float *>(w.g.L);  // the staged basis is consumed before the first factorization
+        w.As32 = w.g.L.as<float>();  // the staged basis is consumed before the first factorization
         w.ldA = m | 1;
         w.s.C = w.g.L;
         w.s.zz = w.g.y;
-        w.s.b = nullptr; w.s.rdiag = nullptr; w.s.posof = nullptr; w.s.zl = nullptr; w.s.diag = nullptr;
+        w.s.b = w.s.rdiag = ShD{0}; w.s.posof = w.s.zl = ShI{0}; w.s.diag = Sh<unsigned char>{0};  // unused
         w.s.lda = lda;
     } else {
-        w.s.C = p; p += (long)lda * n;
+        w.s.C = p; p += lda * n;
         w.s.b = p; p += lda;
         w.s.zz = p; p += lda;
         w.data = p; p += lda;
@@ -52,10 +52,10 @@ static __device__ void warp_setup(Warp &w, const Params &P, double *p, double *s
         w.xout = p; p += n;
         w.s.rdiag = p; p += n;
         p += 8;
-        w.s.idx = reinterpret_cast<int *>(p);
+        w.s.idx = p.as<int>();
         w.s.posof = w.s.idx + n;
         w.s.zl = w.s.posof + n;
-        w.s.diag = reinterpret_cast<unsigned char *>(w.s.zl + 2 * n);
+        w.s.diag = (w.s.zl + 2 * n).as<unsigned char>();
         w.s.lda = lda;
     }
     w.scr = scr;
@@ -69,13 +69,12 @@ static __device__ void warp_setup(Warp &w, const Params &P, double *p, double *s
 // blockDim.x / 32 warps per block, each with its own workspace.  P.mixed
 // selects the method (warp-uniform for the whole launch).
 __device__ __forceinline__ void voxels_body(const Params &P) {
-    extern __shared__ double smem[];
     const int wib = threadIdx.x >> 5, wpb = blockDim.x >> 5;
     Warp w;
     w.lane = threadIdx.x & 31;
     w.nnls_caps = 0;
     w.loop_caps = 0;
-    warp_setup(w, P, smem + (long)wib * P.smem_stride, P.scratch + ((long)blockIdx.x * wpb + wib) * P.scr_stride);
+    warp_setup(w, P, ShD{0} + (int)(wib * P.smem_stride), P.scratch + ((long)blockIdx.x * wpb + wib) * P.scr_stride);
 #if DECAES_TC_PRODUCTS
     // one chunk of the voxel list: positions [tq0, min(tq1, *nvox))
     const long nvox = P.tq1 > 0 && P.tq1 < (long)*P.nvox ? P.tq1 : (long)*P.nvox;
@@ -110,11 +109,9 @@ __device__ __forceinline__ void voxels_body(const Params &P) {
 // copies that volume's parameters next to its workspace and re-carves the
 // workspace for the volume's (nTE, nT2, method).
 __device__ __forceinline__ void voxels_batch_body(const BatchParams &B) {
-    extern __shared__ double smem[];
     const int wib = threadIdx.x >> 5, wpb = blockDim.x >> 5;
-    double *base = smem + (long)wib * B.smem_stride;
-    Params *Pw = reinterpret_cast<Params *>(base);
-    double *ws = base + kParamsDoubles;
+    const ShD base = ShD{0} + (int)(wib * B.smem_stride), ws = base + kParamsDoubles;
+    Params *Pw = reinterpret_cast<Params *>(base.ptr());
     double *scr = B.scratch + ((long)blockIdx.x * wpb + wib) * B.scr_stride;
     Warp w;
     w.lane = threadIdx.x & 31;
