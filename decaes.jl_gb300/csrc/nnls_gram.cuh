@@ -45,6 +45,7 @@ __device__ __forceinline__ int gidx(int i, int j) { return i <= j ? tri(j) + i :
 struct GramWS {
     ShD G;     // packed upper triangle of the Gram matrix, n(n+1)/2
     ShD L;     // packed strictly-lower unit factor of H_PP = L D L'
+    int nL;    // doubles at L
     ShD f;     // A'b
     ShD y;     // L^{-1} f_P
     ShD dd;    // pivots D (during a factorization: the running diagonal)
@@ -197,13 +198,108 @@ static __device__ __noinline__ void gram_load(GramWS &g, const double *Gg, int n
     __syncwarp();
 }
 
-// LDL' factorization of H_PP = G_PP + mu2 I from scratch (right-looking),
-// with y = L^{-1} f_P carried along as an extra column.  Per pivot: one
+// Tile of the factorization: the lower triangle of the matrix still to be
+// factored with the right-hand side as a row below it, in one run of shared
+// memory.  Rows and columns count from the end -- rho = k - r for matrix row r,
+// 0 for the right-hand side; gamma = k - c -- and element (rho, gamma), rho <=
+// gamma, has number gamma (gamma + 1) / 2 + rho.  So the trailing elements of
+// every step, of any k, are the first numbers.  gamma of a number is the count
+// of triangular numbers up to it: those before its block of 32 numbers, and a
+// bit mask of those in the block (one constant load, one population count).
+struct TileBlocks {
+    unsigned mask[66];  // triangular numbers in block s, and how many (of 1, 3, 6, ...) come before it
+    int below[66];
+    constexpr TileBlocks() : mask(), below() {
+        for (int s = 0; s < 66; ++s)
+            for (int g = 1; g * (g + 1) / 2 < 32 * s + 32; ++g)
+                if (g * (g + 1) / 2 < 32 * s) below[s] = g;
+                else mask[s] |= 1u << (g * (g + 1) / 2 - 32 * s);
+    }
+};
+static __constant__ const TileBlocks kTile;
+// element e = 32 s + lane
+__device__ __forceinline__ void tile_element(int s, int e, unsigned lanes_le, int &rho, int &gamma) {
+    gamma = kTile.below[s] + __popc(kTile.mask[s] & lanes_le);
+    rho = e - tri(gamma);
+}
+
+// LDL' factorization of H_PP = G_PP + mu2 I from scratch (right-looking) for k
+// <= 32, with y = L^{-1} f_P carried along as an extra row, on a tile held
+// behind the factor (k^2 doubles for both).  Per pivot: one reciprocal, the
+// column scaled by the lanes of its rows, and the trailing update of 32 tile
+// elements at a time; the elements of the next pivot column also go to a
+// buffer of their own.  gram_refactor_large's update finds each element's row
+// and column by a square root and both operands in the packed factor, ~45
+// instructions a round against ~16 here.  The loops are kept small on purpose:
+// the same tile held in registers (no loads or stores of its elements, 15-30
+// KB of unrolled code) ran 3-35% slower, all of the kernel with it, waiting for
+// instructions.  Returns false when a pivot is not positive relative to its
+// diagonal (numerically dependent set).  Until the results are written, y and
+// dd hold a pivot column and its scaled copy.
+static __device__ __noinline__ bool gram_refactor_tile(const GramWS g, int k, double mu2) {
+    const int lane = threadIdx.x & 31;
+    ShD col = g.xp, nxt = g.y;
+    const ShD lb = g.dd, Lr = g.L + tri(lane - 1), T = g.L + tri(k - 1);
+    double th = 0.0, yv = 0.0, dv = 0.0;  // lane r: row r's pivot threshold tol * H_rr, y and reciprocal pivot
+    if (lane < k) {
+        const int p = g.P[lane];
+        th = kGramDepTol * (g.G[tri(p) + p] + mu2);
+    }
+    const unsigned lanes_le = (2u << lane) - 1u;
+    #pragma unroll 1
+    for (int s = 0, e = lane; e < tri(k + 1); ++s, e += 32) {  // the first pivot column goes to its buffer
+        int rho, gamma;
+        tile_element(s, e, lanes_le, rho, gamma);
+        if (gamma == 0) continue;  // (0, 0) is no element
+        const int pc = g.P[k - gamma];
+        double h;
+        if (rho == 0) {
+            h = g.f[pc];
+        } else {
+            h = g.G[gidx(g.P[k - rho], pc)];
+            if (rho == gamma) h = h + mu2;
+        }
+        if (gamma == k) col[rho] = h;
+        else T[e] = h;
+    }
+    __syncwarp();
+    #pragma unroll 1
+    for (int gp = k; gp > 0; --gp) {  // gamma of the pivot column j = k - gp
+        const int j = k - gp;
+        const double d = col[gp];
+        if (__any_sync(FULL, lane == j && !gt_nonneg_bits(d, th))) return false;  // d > tol * H_jj
+        const double rd = fast_rcp(d);
+        if (lane == j) { yv = col[0]; dv = rd; }
+        if (lane > j && lane < k) {
+            const double l = col[k - lane] * rd;
+            lb[k - lane] = l;
+            Lr[j] = l;
+        }
+        __syncwarp();
+        const int trail = gp > 1 ? tri(gp) : 0;
+        #pragma unroll 1
+        for (int s = 0, e = lane; e < trail; ++s, e += 32) {
+            int rho, gamma;
+            tile_element(s, e, lanes_le, rho, gamma);
+            const double h = fma(-col[rho], lb[gamma], T[e]);
+            T[e] = h;
+            if (gamma == gp - 1) nxt[rho] = h;
+        }
+        const ShD s = col; col = nxt; nxt = s;
+        __syncwarp();
+    }
+    if (lane < k) { g.y[lane] = yv; g.dinv[lane] = dv; }
+    __syncwarp();
+    return true;
+}
+
+// LDL' factorization of H_PP = G_PP + mu2 I from scratch (right-looking)
+// for any k, with y = L^{-1} f_P carried along as an extra column.  Per pivot: one
 // reciprocal, the column scaled by the lanes of its rows, and the trailing
 // update -- diagonal included -- spread over lanes by (row, column) pair, so a
 // step costs ~(k-j)^2/64 FMA instructions instead of k-j.  Returns false when
 // a pivot is not positive relative to its diagonal (numerically dependent set).
-static __device__ __noinline__ bool gram_refactor(GramWS g, int k, double mu2) {
+static __device__ __noinline__ bool gram_refactor_large(GramWS g, int k, double mu2) {
     const int lane = threadIdx.x & 31;
     const int r0 = lane, r1 = lane + 32;
     const int p0 = r0 < k ? g.P[r0] : 0, p1 = r1 < k ? g.P[r1] : 0;
@@ -266,6 +362,10 @@ static __device__ __noinline__ bool gram_refactor(GramWS g, int k, double mu2) {
     if (r1 < k) g.y[r1] = v1;
     __syncwarp();
     return true;
+}
+
+__device__ __forceinline__ bool gram_refactor(const GramWS &g, int k, double mu2) {
+    return k <= 32 && k * k <= g.nL ? gram_refactor_tile(g, k, mu2) : gram_refactor_large(g, k, mu2);
 }
 
 // Extends the factorization by column t (k -> k+1): u = L^{-1} H[P,t],

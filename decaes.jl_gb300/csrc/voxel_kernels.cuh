@@ -23,7 +23,7 @@ static __device__ void warp_setup(Warp &w, const Params &P, ShD p, double *scr) 
         w.s.w = p; p += n;
         w.xout = p; p += n;
         w.g.G = p; p += (int)mixed_r1_doubles(m, n);
-        w.g.L = p; p += (int)mixed_r2_doubles(m, n, P.reg == 2);
+        w.g.L = p; p += w.g.nL = (int)mixed_r2_doubles(m, n, P.reg == 2);
         w.g.f = p; p += n;
         w.g.y = p; p += n;
         w.g.dd = p; p += n;
