@@ -48,32 +48,28 @@ struct GramWS {
     int nL;    // doubles at L
     ShD f;     // A'b
     ShD y;     // L^{-1} f_P
-    ShD dd;    // pivots D (during a factorization: the running diagonal)
+    ShD dd;    // factorization scratch: the running diagonal, or a scaled pivot column
     ShD dinv;  // 1 / D
     ShD xp;    // x on P (xp[r] = x[P[r]])
-    ShI P;        // passive columns, 0-based, k entries
-    ShI pos;      // pos[j] = index of column j in P, or -1
-    ShI lastP;    // passive set left by the previous solve (warm start)
+    ShI P;     // passive columns, 0-based, k entries; kept for the next solve's warm start
     int lastk;
     double bb;     // b'b
 };
 
-// Warp-wide maximum (minimum) of integer keys; ties go to the smaller index.
-__device__ __forceinline__ void warp_keymax(long long &key, int &j) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        long long ok = __shfl_xor_sync(FULL, key, o);
-        int oj = __shfl_xor_sync(FULL, j, o);
-        if (ok > key || (ok == key && oj < j)) { key = ok; j = oj; }
-    }
+// Warp-wide maximum of the bit patterns of non-negative doubles (0: no entry)
+// and the smallest index j that holds it; warp_bitsmin likewise the minimum.
+// Three integer warp reductions instead of a butterfly's fifteen shuffles.
+__device__ __forceinline__ unsigned long long warp_bitsmax(unsigned long long v, int &j) {
+    const unsigned hi = (unsigned)(v >> 32), lo = (unsigned)v;
+    const unsigned mh = __reduce_max_sync(FULL, hi), ml = __reduce_max_sync(FULL, hi == mh ? lo : 0u);
+    j = (int)__reduce_min_sync(FULL, hi == mh && lo == ml ? (unsigned)j : 0xffffffffu);
+    return (unsigned long long)mh << 32 | ml;
 }
-__device__ __forceinline__ void warp_keymin(long long &key, int &j) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        long long ok = __shfl_xor_sync(FULL, key, o);
-        int oj = __shfl_xor_sync(FULL, j, o);
-        if (ok < key || (ok == key && oj < j)) { key = ok; j = oj; }
-    }
+__device__ __forceinline__ unsigned long long warp_bitsmin(unsigned long long v, int &j) {
+    const unsigned hi = (unsigned)(v >> 32), lo = (unsigned)v;
+    const unsigned mh = __reduce_min_sync(FULL, hi), ml = __reduce_min_sync(FULL, hi == mh ? lo : 0xffffffffu);
+    j = (int)__reduce_min_sync(FULL, hi == mh && lo == ml ? (unsigned)j : 0xffffffffu);
+    return (unsigned long long)mh << 32 | ml;
 }
 
 // 1/d for normal d: the hardware's approximate FP64 reciprocal (rcp.approx,
@@ -373,16 +369,26 @@ __device__ __forceinline__ bool gram_refactor(const GramWS &g, int k, double mu2
 // not positive relative to H_tt or when its coefficient y_t / delta in the
 // unconstrained solution on P + {t} is not positive (the guards of the
 // reference's Householder step).  Returns true when t was added.
-static __device__ __noinline__ bool gram_append(GramWS g, int k, int t, double mu2) {
+static __device__ __noinline__ bool gram_append(const GramWS g, int k, int t, double mu2) {
     const int lane = threadIdx.x & 31;
     const int r0 = lane, r1 = lane + 32;
-    const ShD L0 = g.L + tri(r0 - 1), L1 = g.L + tri(r1 - 1);
-    double v0 = r0 < k ? g.G[gidx(g.P[r0], t)] : 0.0, v1 = r1 < k ? g.G[gidx(g.P[r1], t)] : 0.0;
-    #pragma unroll 1
-    for (int i = 0; i < k; ++i) {
-        const double ui = lane_pick(v0, v1, i);
-        if (r0 > i && r0 < k) v0 = fma(-L0[i], ui, v0);
-        if (r1 > i && r1 < k) v1 = fma(-L1[i], ui, v1);
+    double v0 = r0 < k ? g.G[gidx(g.P[r0], t)] : 0.0, v1 = 0.0;
+    const ShD L0 = g.L + tri(r0 - 1);
+    if (k <= 32) {
+        #pragma unroll 1
+        for (int i = 0; i < k; ++i) {
+            const double ui = bcast(v0, i);
+            if (r0 > i && r0 < k) v0 = fma(-L0[i], ui, v0);
+        }
+    } else {
+        const ShD L1 = g.L + tri(r1 - 1);
+        if (r1 < k) v1 = g.G[gidx(g.P[r1], t)];
+        #pragma unroll 1
+        for (int i = 0; i < k; ++i) {
+            const double ui = lane_pick(v0, v1, i);
+            if (r0 > i) v0 = fma(-L0[i], ui, v0);
+            if (r1 > i && r1 < k) v1 = fma(-L1[i], ui, v1);
+        }
     }
     double w0 = 0.0, w1 = 0.0, pl = 0.0, py = 0.0;
     if (r0 < k) { w0 = v0 * g.dinv[r0]; pl = fma(v0, w0, pl); py = fma(w0, g.y[r0], py); }
@@ -398,11 +404,9 @@ static __device__ __noinline__ bool gram_append(GramWS g, int k, int t, double m
     if (r0 < k) Lk[r0] = w0;
     if (r1 < k) Lk[r1] = w1;
     if (lane == 0) {
-        g.dd[k] = delta;
         g.dinv[k] = fast_rcp(delta);
         g.y[k] = yt;
         g.P[k] = t;
-        g.pos[t] = k;
     }
     __syncwarp();
     return true;
@@ -413,13 +417,22 @@ static __device__ __noinline__ bool gram_append(GramWS g, int k, int t, double m
 static __device__ __noinline__ double2 gram_back(const GramWS g, int k) {
     const int lane = threadIdx.x & 31;
     const int r0 = lane, r1 = lane + 32;
-    double u0 = r0 < k ? g.y[r0] * g.dinv[r0] : 0.0, u1 = r1 < k ? g.y[r1] * g.dinv[r1] : 0.0;
+    double u0 = r0 < k ? g.y[r0] * g.dinv[r0] : 0.0, u1 = 0.0;
+    int i = k - 1;
+    if (k > 32) {
+        if (r1 < k) u1 = g.y[r1] * g.dinv[r1];
+        #pragma unroll 1
+        for (; i >= 32; --i) {
+            const double zi = bcast(u1, i & 31);
+            const ShD Li = g.L + tri(i - 1);
+            u0 = fma(-Li[r0], zi, u0);
+            if (r1 < i) u1 = fma(-Li[r1], zi, u1);
+        }
+    }
     #pragma unroll 1
-    for (int i = k - 1; i >= 0; --i) {
-        const double zi = lane_pick(u0, u1, i);
-        const ShD Li = g.L + tri(i - 1);
-        if (r0 < i) u0 = fma(-Li[r0], zi, u0);
-        if (r1 < i) u1 = fma(-Li[r1], zi, u1);
+    for (; i > 0; --i) {
+        const double zi = bcast(u0, i);
+        if (r0 < i) u0 = fma(-g.L[tri(i - 1) + r0], zi, u0);
     }
     return make_double2(u0, u1);
 }
@@ -571,199 +584,143 @@ static __device__ __noinline__ void gram_svdvals(GramWS g, const ShD W, int m, i
 
 // NNLS on H = G + mu2 I with right-hand side f (prepared by gram_rhs_t /
 // gram_build_f32 / gram_load, which also set b'b).  On return x (dense, n)
-// holds the solution, idx its passive columns (1-based, nsetp entries) and
-// rnorm^2 = ||A x - b||^2 + mu2 ||x||^2.  mode = 1 when max_iter was reached
-// (the reference's cap 3n).
-static __device__ __noinline__ NnlsResult gram_nnls(GramWS g, const ShD x, const ShD wv, const ShI idx, int n, double mu2,
+// holds the solution, nsetp the size of its passive set (in g.P, from where
+// the next solve of the voxel starts: *lastk_io entries, 0: from scratch),
+// rnorm^2 = ||A x - b||^2 + mu2 ||x||^2 and xx = ||x||^2 as warp_seminorm_sq
+// sums it.  mode = 1 when max_iter was reached (the reference's cap 3n).
+//
+// x on the passive set lives on the lanes of its rows (x0, x1); the free
+// columns' duals, compacted, in wv with their columns in fc.
+static __device__ __noinline__ NnlsResult gram_nnls(const GramWS g, const ShD x, const ShD wv, const ShI fc, int n, double mu2,
                                              int max_iter, int *lastk_io) {
     const int lane = threadIdx.x & 31;
     const int r0 = lane, r1 = lane + 32;
-    #pragma unroll 1
-    for (int j = lane; j < n; j += 32) { x[j] = 0.0; g.pos[j] = -1; }
-    __syncwarp();
-    int k = 0, iters = 0, mode = 0;
-
+    const unsigned below = (1u << lane) - 1u;
+    double x0 = 0.0, x1 = 0.0;
+    int k = *lastk_io, nf = 0, iters = 0, mode = 0;
     // warm start: the previous passive set, pruned until its unconstrained
     // solution is positive
-    const int lastk = *lastk_io;
-    if (lastk > 0) {
-        #pragma unroll 1
-        for (int r = lane; r < lastk; r += 32) { g.P[r] = g.lastP[r]; g.pos[g.lastP[r]] = r; }
-        __syncwarp();
-        k = lastk;
-        #pragma unroll 1
-        for (int round = 0; round < kGramMaxN && k > 0; ++round) {
-            if (!gram_refactor(g, k, mu2)) {
-                #pragma unroll 1
-                for (int r = lane; r < k; r += 32) g.pos[g.P[r]] = -1;
-                __syncwarp();
-                k = 0;
-                break;
-            }
-            const double2 zz = gram_back(g, k);
-            const double z0 = zz.x, z1 = zz.y;
-            const bool keep0 = r0 < k && pos_bits(z0), keep1 = r1 < k && pos_bits(z1);
-            const unsigned m0 = __ballot_sync(FULL, keep0), m1 = __ballot_sync(FULL, keep1);
-            const int kk = __popc(m0) + __popc(m1);
-            if (kk == k) {
-                if (r0 < k) x[g.P[r0]] = z0;
-                if (r1 < k) x[g.P[r1]] = z1;
-                __syncwarp();
-                break;
-            }
-            // compact P to the positive coefficients
-            const int p0 = r0 < k ? g.P[r0] : -1, p1 = r1 < k ? g.P[r1] : -1;
-            __syncwarp();
-            const unsigned below = (1u << lane) - 1u;
-            if (r0 < k) {
-                if (keep0) { int d = __popc(m0 & below); g.P[d] = p0; g.pos[p0] = d; }
-                else g.pos[p0] = -1;
-            }
-            if (r1 < k) {
-                if (keep1) { int d = __popc(m0) + __popc(m1 & below); g.P[d] = p1; g.pos[p1] = d; }
-                else g.pos[p1] = -1;
-            }
-            __syncwarp();
-            k = kk;
-        }
-    }
-
-    unsigned long long rejected = 0ull;  // columns refused since the last change of P (warp-uniform)
-    bool dual_stale = true;
+    bool warm = k > 0, dual_stale = true;
+    unsigned long long rejected = 0ull;  // free columns (positions in fc) refused since the last change of P
     #pragma unroll 1
-    for (int outer = 0;; ++outer) {
-        if (outer > 4 * max_iter) { mode = 1; break; }
-        // dual w_j = f_j - sum_r G[j, P_r] x_{P_r} on the non-passive columns
-        if (dual_stale) {
-            #pragma unroll 1
-            for (int r = lane; r < k; r += 32) g.xp[r] = x[g.P[r]];
-            // the free columns in column order, compacted into idx (free until
-            // the outputs), so that up to 32 of them take one round of lanes
-            // (only free columns' duals are read)
-            const bool fr0 = r0 < n && g.pos[r0] < 0, fr1 = r1 < n && g.pos[r1] < 0;
-            const unsigned b0 = __ballot_sync(FULL, fr0), b1 = __ballot_sync(FULL, fr1);
-            const unsigned below = (1u << lane) - 1u;
-            if (fr0) idx[__popc(b0 & below)] = r0;
-            if (fr1) idx[__popc(b0) + __popc(b1 & below)] = r1;
-            const int nf = __popc(b0) + __popc(b1);
-            __syncwarp();
+    for (int outer = warm ? -1 : 0;; ++outer) {
+        if (!warm) {
+            if (outer > 4 * max_iter) { mode = 1; break; }
+            // dual w_j = f_j - sum_r G[j, P_r] x_{P_r} on the free columns j: in
+            // column order, so that up to 32 of them take one round of lanes
+            if (dual_stale) {
+                const int p0 = r0 < k ? g.P[r0] : -1, p1 = r1 < k ? g.P[r1] : -1;
+                unsigned in0 = 0u, in1 = 0u;  // passive columns 0-31, 32-63
+                if (p0 >= 0) { if (p0 < 32) in0 = 1u << p0; else in1 = 1u << (p0 - 32); }
+                if (p1 >= 0) { if (p1 < 32) in0 |= 1u << p1; else in1 |= 1u << (p1 - 32); }
+                in0 = __reduce_or_sync(FULL, in0);
+                in1 = __reduce_or_sync(FULL, in1);
+                const unsigned b0 = ~in0 & (n >= 32 ? ~0u : (1u << n) - 1u), b1 = n > 32 ? ~in1 & (~0u >> (64 - n)) : 0u;
+                if (b0 >> lane & 1u) fc[__popc(b0 & below)] = r0;
+                if (b1 >> lane & 1u) fc[__popc(b0) + __popc(b1 & below)] = r1;
+                nf = __popc(b0) + __popc(b1);
+                if (r0 < k) g.xp[r0] = x0;
+                if (r1 < k) g.xp[r1] = x1;
+                __syncwarp();
+                #pragma unroll 1
+                for (int i = lane; i < nf; i += 32) {
+                    const int j = fc[i];
+                    double s = g.f[j], s2 = 0.0;
+                    int r = 0;
+                    #pragma unroll 1
+                    for (; r + 1 < k; r += 2) {
+                        s = fma(-g.G[gidx(j, g.P[r])], g.xp[r], s);
+                        s2 = fma(-g.G[gidx(j, g.P[r + 1])], g.xp[r + 1], s2);
+                    }
+                    if (r < k) s = fma(-g.G[gidx(j, g.P[r])], g.xp[r], s);
+                    wv[i] = s + s2;
+                }
+                __syncwarp();
+                dual_stale = false;
+            }
+            if (k >= n) break;
+            // entering column: largest positive dual among the unrefused ones, first column on ties
+            unsigned long long best = 0;
+            int bi = 0;
             #pragma unroll 1
             for (int i = lane; i < nf; i += 32) {
-                const int j = idx[i];
-                double s = g.f[j], s2 = 0.0;
-                int r = 0;
-                #pragma unroll 1
-                for (; r + 1 < k; r += 2) {
-                    s = fma(-g.G[gidx(j, g.P[r])], g.xp[r], s);
-                    s2 = fma(-g.G[gidx(j, g.P[r + 1])], g.xp[r + 1], s2);
-                }
-                if (r < k) s = fma(-g.G[gidx(j, g.P[r])], g.xp[r], s);
-                wv[j] = s + s2;
+                const double w = wv[i];
+                const unsigned long long key = (unsigned long long)__double_as_longlong(w);
+                if (pos_bits(w) && !(rejected >> i & 1ull) && key > best) { best = key; bi = i; }
             }
-            __syncwarp();
-            dual_stale = false;
+            best = warp_bitsmax(best, bi);
+            if (best == 0) break;
+            if (!gram_append(g, k, fc[bi], mu2)) {
+                rejected |= 1ull << bi;
+                continue;
+            }
+            if (r0 == k) x0 = 0.0;
+            if (r1 == k) x1 = 0.0;
+            k += 1;
+            rejected = 0ull;
         }
-        if (k >= n) break;
-        // entering column: largest positive dual among free, unrefused columns
-        long long best = -1;
-        int bj = 0x7fffffff;
-        #pragma unroll 1
-        for (int j = lane; j < n; j += 32) {
-            if (g.pos[j] >= 0 || ((rejected >> j) & 1ull)) continue;
-            const double wj = wv[j];
-            if (!pos_bits(wj)) continue;
-            const long long key = okey(wj);
-            if (key > best) { best = key; bj = j; }
-        }
-        warp_keymax(best, bj);
-        if (best < 0) break;
-        if (!gram_append(g, k, bj, mu2)) {
-            rejected |= 1ull << bj;
-            continue;
-        }
-        k += 1;
-        rejected = 0ull;
-        // inner loop: move toward the unconstrained solution on P
+        // move toward the unconstrained solution on P (a warm start: drop the
+        // columns whose coefficients in it are not positive)
+        bool factored = !warm;
         #pragma unroll 1
         for (;;) {
+            if (!factored && !gram_refactor(g, k, mu2)) { k = 0; break; }  // numerically dependent: from the empty set
             const double2 zz = gram_back(g, k);
             const double z0 = zz.x, z1 = zz.y;
             const bool pos0 = !(r0 < k) || pos_bits(z0), pos1 = !(r1 < k) || pos_bits(z1);
-            if (__all_sync(FULL, pos0 && pos1)) {
-                if (r0 < k) x[g.P[r0]] = z0;
-                if (r1 < k) x[g.P[r1]] = z1;
-                __syncwarp();
-                break;
+            if (__all_sync(FULL, pos0 && pos1)) { x0 = z0; x1 = z1; break; }
+            double nx0 = z0, nx1 = z1;
+            if (!warm) {
+                if (++iters > max_iter) { mode = 1; break; }
+                // alpha = min over z_r <= 0 of x_r / (x_r - z_r), first row on ties (bit
+                // patterns of non-negative values order like the values)
+                double a0 = CUDART_INF, a1 = CUDART_INF;
+                if (!pos0) { const double dz = x0 - z0; a0 = pos_bits(dz) ? x0 * fast_rcp(dz) : 0.0; }
+                if (!pos1) { const double dz = x1 - z1; a1 = pos_bits(dz) ? x1 * fast_rcp(dz) : 0.0; }
+                unsigned long long ka = (unsigned long long)__double_as_longlong(a0);
+                const unsigned long long ka1 = (unsigned long long)__double_as_longlong(a1);
+                int ia = r0;
+                if (ka1 < ka) { ka = ka1; ia = r1; }
+                const double alpha = __longlong_as_double((long long)warp_bitsmin(ka, ia));
+                nx0 = r0 == ia ? 0.0 : fma(alpha, z0 - x0, x0);
+                nx1 = r1 == ia ? 0.0 : fma(alpha, z1 - x1, x1);
             }
-            if (++iters > max_iter) { mode = 1; break; }
-            // alpha = min over z_r <= 0 of x_r / (x_r - z_r)
-            double a0 = CUDART_INF, a1 = CUDART_INF;
-            const double x0 = r0 < k ? x[g.P[r0]] : 0.0, x1 = r1 < k ? x[g.P[r1]] : 0.0;
-            if (r0 < k && !pos_bits(z0)) { const double dz = x0 - z0; a0 = pos_bits(dz) ? x0 * fast_rcp(dz) : 0.0; }
-            if (r1 < k && !pos_bits(z1)) { const double dz = x1 - z1; a1 = pos_bits(dz) ? x1 * fast_rcp(dz) : 0.0; }
-            const long long ka0 = okey(a0), ka1 = okey(a1);  // a0, a1 are not NaN: min without the FP64 pipe
-            long long ka = ka0 <= ka1 ? ka0 : ka1;
-            int ia = ka0 <= ka1 ? r0 : r1;
-            warp_keymin(ka, ia);
-            const double alpha = lane_pick(a0, a1, ia);
-            double nx0 = x0, nx1 = x1;
-            if (r0 < k) nx0 = fma(alpha, z0 - x0, x0);
-            if (r1 < k) nx1 = fma(alpha, z1 - x1, x1);
-            if (r0 == ia) nx0 = 0.0;
-            if (r1 == ia) nx1 = 0.0;
             const bool keep0 = r0 < k && pos_bits(nx0), keep1 = r1 < k && pos_bits(nx1);
             const unsigned m0 = __ballot_sync(FULL, keep0), m1 = __ballot_sync(FULL, keep1);
-            const int p0 = r0 < k ? g.P[r0] : -1, p1 = r1 < k ? g.P[r1] : -1;
+            const int p0 = r0 < k ? g.P[r0] : 0, p1 = r1 < k ? g.P[r1] : 0;
             __syncwarp();
-            const unsigned below = (1u << lane) - 1u;
-            if (r0 < k) {
-                x[p0] = keep0 ? nx0 : 0.0;
-                if (keep0) { int d = __popc(m0 & below); g.P[d] = p0; g.pos[p0] = d; }
-                else g.pos[p0] = -1;
-            }
-            if (r1 < k) {
-                x[p1] = keep1 ? nx1 : 0.0;
-                if (keep1) { int d = __popc(m0) + __popc(m1 & below); g.P[d] = p1; g.pos[p1] = d; }
-                else g.pos[p1] = -1;
-            }
-            __syncwarp();
+            if (keep0) { const int d = __popc(m0 & below); g.P[d] = p0; g.xp[d] = nx0; }
+            if (keep1) { const int d = __popc(m0) + __popc(m1 & below); g.P[d] = p1; g.xp[d] = nx1; }
             k = __popc(m0) + __popc(m1);
-            if (!gram_refactor(g, k, mu2)) {
-                // numerically dependent remainder: restart from the empty set
-                #pragma unroll 1
-                for (int r = lane; r < k; r += 32) { g.pos[g.P[r]] = -1; x[g.P[r]] = 0.0; }
-                __syncwarp();
-                k = 0;
-            }
+            __syncwarp();
+            if (r0 < k) x0 = g.xp[r0];
+            if (r1 < k) x1 = g.xp[r1];
+            __syncwarp();
+            factored = false;
         }
-        dual_stale = true;
         if (mode) break;
+        warm = false;
+        dual_stale = true;
     }
 
-    // outputs: passive list, warm-start set, residual
-    #pragma unroll 1
-    for (int r = lane; r < k; r += 32) { idx[r] = g.P[r] + 1; g.lastP[r] = g.P[r]; }
     *lastk_io = k;
-    __syncwarp();
     #pragma unroll 1
-    for (int r = lane; r < k; r += 32) g.xp[r] = x[g.P[r]];
+    for (int j = lane; j < n; j += 32) x[j] = 0.0;
     __syncwarp();
     // ||A x - b||^2 = b'b - f'x - mu^2 ||x||^2 at the solution ((G + mu^2 I)_PP x_P
     // = f_P); the cancellation costs ~eps * b'b, far below the noise floor
     double fx = 0.0, xx = 0.0;
-    #pragma unroll 1
-    for (int r = lane; r < k; r += 32) {
-        const double xr = g.xp[r];
-        fx = fma(g.f[g.P[r]], xr, fx);
-        xx = fma(xr, xr, xx);
-    }
+    if (r0 < k) { const int p = g.P[r0]; x[p] = x0; fx = fma(g.f[p], x0, 0.0); xx = x0 * x0; }
+    double xs = xx;
+    if (r1 < k) { const int p = g.P[r1]; x[p] = x1; fx = fma(g.f[p], x1, fx); xx = fma(x1, x1, xx); xs = xs + x1 * x1; }
     wsum2(fx, xx, fx, xx);  // the same pairings as wsum, both sums in one butterfly
     const double res = fmax(g.bb - fx - mu2 * xx, 0.0);
     NnlsResult out;
     out.nsetp = k;
     out.mode = mode;
     out.rnorm = sqrt(fma(mu2, xx, res));
-    out.xx = xx;
+    out.xx = k <= 32 ? xx : wsum(xs);  // (one term per lane: the same sum)
+    __syncwarp();
     return out;
 }
 

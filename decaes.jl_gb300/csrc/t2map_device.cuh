@@ -155,10 +155,9 @@ static __device__ TikhState tikh_solve(Warp &w, double mu) {
 static __device__ double tikh_res2_ssq(const TikhState &t, double ssq) {
     return jmax(__dsub_rn(__dmul_rn(t.r.rnorm, t.r.rnorm), __dmul_rn(__dmul_rn(t.mu, t.mu), ssq)), 0.0);
 }
-// ||x||^2 of the solution just computed.  The mixed solver has summed it: with
-// one term per lane its sum is warp_seminorm_sq's, bit for bit.
+// ||x||^2 of the solution just computed (the mixed solver has summed it).
 static __device__ double solution_ssq(Warp &w, const TikhState &t) {
-    return use_mixed(w) && t.r.nsetp <= 32 ? t.r.xx : warp_seminorm_sq(w.s, t.r.nsetp);
+    return use_mixed(w) ? t.r.xx : warp_seminorm_sq(w.s, t.r.nsetp);
 }
 static __device__ double tikh_res2(Warp &w, const TikhState &t) { return tikh_res2_ssq(t, solution_ssq(w, t)); }
 static __device__ void save_x(Warp &w) {
@@ -1093,10 +1092,11 @@ static __device__ DK_OUTLINE void fa_suggest(Search &S, double &xo, double &uo) 
                 hermite_minimize(g[Il], g[Ir], S.u[Il], S.u[Ir], S.du[Il], S.du[Ir], x, v);
             }
             __syncwarp();
-            long long key = isnan_bits(v) ? LLONG_MAX : okey(v);
+            // okey with its sign flipped orders as unsigned; a NaN never wins
             int i = lane;
-            warp_keymin(key, i);
-            if (key < okey(u)) { p = bcast(x, i); u = bcast(v, i); }
+            const unsigned long long flip = 1ull << 63;
+            const unsigned long long key = warp_bitsmin(isnan_bits(v) ? ~0ull : (unsigned long long)okey(v) ^ flip, i);
+            if (key < ((unsigned long long)okey(u) ^ flip)) { p = bcast(x, i); u = bcast(v, i); }
         }
     }
     xo = p;

@@ -88,7 +88,7 @@ __host__ __device__ inline long mixed_r2_doubles(int m, int n, bool gcv) {
 }
 __host__ __device__ inline long warp_smem_doubles_mixed(int m, int n, bool gcv) {
     long d = (long)m + 3L * n + mixed_r1_doubles(m, n) + mixed_r2_doubles(m, n, gcv) + 5L * n + 8;
-    long ints = 4L * n;  // idx, P, pos, lastP
+    long ints = 2L * n;  // idx, P
     return d + (ints * 4 + 7) / 8;
 }
 // Lanes of the FP64 method's EPG basis (one T2 column per lane, 3m states

@@ -33,8 +33,6 @@ static __device__ void warp_setup(Warp &w, const Params &P, ShD p, double *scr) 
         const ShI ip = p.as<int>();
         w.s.idx = ip;
         w.g.P = ip + n;
-        w.g.pos = ip + 2 * n;
-        w.g.lastP = ip + 3 * n;
         w.g.lastk = 0;
         w.As32 = w.g.L.as<float>();  // the staged basis is consumed before the first factorization
         w.ldA = m | 1;
