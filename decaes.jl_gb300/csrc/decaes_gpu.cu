@@ -138,10 +138,10 @@ __global__ void __launch_bounds__(128) k_voxels_batch(const __grid_constant__ Ba
 __global__ void __launch_bounds__(128) k_voxels_legacy(const __grid_constant__ Params P);
 __global__ void __launch_bounds__(128) k_voxels_batch_legacy(const __grid_constant__ BatchParams B);
 __global__ void __launch_bounds__(256) k_voxels_plain(const __grid_constant__ Params P);
-__global__ void __launch_bounds__(128) k_voxels_mixed(const __grid_constant__ Params P);
-__global__ void __launch_bounds__(128) k_voxels_mixed_tc(const __grid_constant__ Params P);
+__global__ void __launch_bounds__(512) k_voxels_mixed(const __grid_constant__ Params P);
+__global__ void __launch_bounds__(512) k_voxels_mixed_tc(const __grid_constant__ Params P);
 __global__ void __launch_bounds__(128) k_voxels_batch_plain(const __grid_constant__ BatchParams B);
-__global__ void __launch_bounds__(128) k_voxels_batch_mixed(const __grid_constant__ BatchParams B);
+__global__ void __launch_bounds__(512) k_voxels_batch_mixed(const __grid_constant__ BatchParams B);
 
 // The batched kernel for a set of volumes: the legacy one when any volume is
 // legacy, else the kernel of the volumes' one method, else the two-method one.
@@ -258,7 +258,7 @@ struct TuneKey {
     }
 };
 struct Tune {
-    int wpb = 1;
+    int wpb = 1;  // 0: the default shape (most resident warps) was the fastest
     int bps = 0;  // resident blocks per SM of the persistent grid (0: as many as fit)
     double us_per_voxel = 0;
 };
@@ -283,6 +283,7 @@ struct decaes_ctx {
     int sms = 0;
     size_t smem_optin = 0;
     std::map<TuneKey, Tune> tune;
+    std::map<std::pair<const void *, long>, int> wpb;  // most_warps_wpb per kernel and workspace
     int force_wpb = 0;  // autotuner trials
     int force_bps = 0;
     int tc_chunks = 0;                 // tensor-core product launches of the last call
@@ -480,7 +481,6 @@ int make_params(decaes_ctx *ctx, const decaes_t2map_opts &o, const dh::T2partPla
     return DECAES_OK;
 }
 
-// Warps per block of the voxel kernel for a problem shape (autotuned, else 1).
 // Warps per block for a launch of these options: forced, else autotuned,
 // else 0 (no preference).
 int tuned_wpb_or0(decaes_ctx *ctx, const decaes_t2map_opts &o) {
@@ -500,17 +500,19 @@ int tuned_bps(decaes_ctx *ctx, const decaes_t2map_opts &o) {
     auto it = ctx->tune.find(k);
     return it == ctx->tune.end() ? 0 : it->second.bps;
 }
-int tuned_wpb(decaes_ctx *ctx, const decaes_t2map_opts &o) {
-    const int w = tuned_wpb_or0(ctx, o);
-    return w > 0 ? w : 1;
-}
 
-// The block size (1..max_wpb warps) that keeps the most warps resident per SM
-// for a kernel whose warps each need `stride` doubles of shared memory (each
-// block also reserves shared memory of its own, so one large block can hold a
-// warp more than single-warp blocks do); ties go to the smaller block.
+// The block size that keeps the most warps resident per SM for a kernel whose
+// warps each need `stride` doubles of shared memory: every block reserves 1 KB
+// of its own besides its warps' workspaces, so one large block can hold a warp
+// or two more than single-warp blocks do (mixed method at 40 T2 times 15
+// instead of 13, at 60 with GCV 7 instead of 6).  Ties go to the smaller block.
 template <class Kern>
-int most_warps_wpb(decaes_ctx *ctx, Kern kern, long stride, int max_wpb) {
+int most_warps_wpb(decaes_ctx *ctx, Kern kern, long stride) {
+    const auto key = std::make_pair((const void *)kern, stride);
+    auto it = ctx->wpb.find(key);
+    if (it != ctx->wpb.end()) return it->second;
+    cudaFuncAttributes at;
+    const int max_wpb = cudaFuncGetAttributes(&at, kern) == cudaSuccess ? at.maxThreadsPerBlock / 32 : 1;
     int best = 1, best_warps = 0;
     for (int w = 1; w <= max_wpb; ++w) {
         const size_t smem = (size_t)w * stride * sizeof(double);
@@ -520,7 +522,15 @@ int most_warps_wpb(decaes_ctx *ctx, Kern kern, long stride, int max_wpb) {
         if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * w, smem) != cudaSuccess) break;
         if (per_sm * w > best_warps) { best_warps = per_sm * w; best = w; }
     }
-    return best;
+    if (ctx->wpb.size() >= 256) ctx->wpb.clear();
+    return ctx->wpb[key] = best;
+}
+// Warps per block of a launch of these options: forced or autotuned, else the
+// most resident warps (legacy kernels: 1).
+template <class Kern>
+int launch_wpb(decaes_ctx *ctx, const decaes_t2map_opts &o, Kern kern, long stride) {
+    if (const int w = tuned_wpb_or0(ctx, o)) return w;
+    return o.legacy ? 1 : most_warps_wpb(ctx, kern, stride);
 }
 
 // Persistent grid for a kernel whose warps each need `stride` doubles of
@@ -588,14 +598,12 @@ int run_t2map(decaes_ctx *ctx, const decaes_t2map_opts &o, const decaes_t2part_o
     // persistent voxel kernel
     P.nvox = d_nvox; P.vidx = (const int *)vidx; P.counter = d_counter; P.stats = d_stats;
     P.smem_stride = wsm;
-    int wpb = tuned_wpb(ctx, o), grid = 0;
+    int grid = 0;
     size_t smem = 0;
     const bool tc = o.precision == DECAES_PREC_MIXED_TC && P.angle_mode == 0 && !o.legacy;
     auto kern = o.legacy ? dk::k_voxels_legacy
                          : (tc ? dk::k_voxels_mixed_tc : (is_mixed(o) ? dk::k_voxels_mixed : dk::k_voxels_plain));
-    // the plain method's large workspace: blocks of up to 8 warps can hold a
-    // warp per SM more than single-warp blocks (its kernel allows 256 threads)
-    if (kern == dk::k_voxels_plain && tuned_wpb_or0(ctx, o) == 0) wpb = most_warps_wpb(ctx, kern, wsm, 8);
+    int wpb = launch_wpb(ctx, o, kern, wsm);
     if (int rc = launch_shape(ctx, kern, wsm, &wpb, &grid, &smem, tuned_bps(ctx, o))) return rc;
     void *scr;
     if (int rc = buf(ctx, "scratch", sizeof(double) * (size_t)P.scr_stride * grid * wpb, &scr)) return rc;
@@ -1159,7 +1167,7 @@ int batch_plan(decaes_ctx *ctx, const decaes_volume *vols, int nvol, cudaStream_
             (is_mixed(o) ? any_mixed : any_plain) = true;
         }
         c.kern = dk::batch_kernel(legacy, any_plain, any_mixed);
-        c.wpb = tuned_wpb(ctx, bp.vols[c.first].v.mopts);
+        c.wpb = launch_wpb(ctx, bp.vols[c.first].v.mopts, c.kern, c.smem_stride);
         if (int rc = launch_shape(ctx, c.kern, c.smem_stride, &c.wpb, &c.grid, &c.smem, tuned_bps(ctx, bp.vols[c.first].v.mopts)))
             return rc;
         bp.scr_doubles = std::max(bp.scr_doubles, c.scr_stride * c.grid * c.wpb);
@@ -1415,7 +1423,8 @@ extern "C" int decaes_autotune(decaes_ctx *ctx, const decaes_t2map_opts *opts, d
     if (int rc = out_layout(ctx, o, false, om)) return rc;
     // Launch shapes tried: warps per block (voxels in flight per block) 1, 2
     // and 4, each with as many resident blocks per SM as fit and with one and
-    // two fewer (fewer warps sharing an SM's FP64 pipes, L1 and L2 share).
+    // two fewer (fewer warps sharing an SM's FP64 pipes, L1 and L2 share); then
+    // the default shape of an untuned call, which stays when it is the fastest.
     const int cand[3] = {1, 2, 4};
     int best_w = 1, best_b = 0;
     double best_ms = 1e30;
@@ -1462,12 +1471,15 @@ extern "C" int decaes_autotune(decaes_ctx *ctx, const decaes_t2map_opts *opts, d
     const bool fixed = !std::isnan(o.SetFlipAngle);
     TuneKey k{o.nTE, o.nT2, fixed ? 1 : o.nRefAngles, o.Reg, is_mixed(o), o.RefConAngle == 180.0,
               o.legacy != 0};
+    ctx->tune.erase(k);
+    float t_default = 0;
+    if (int rc = trial(0, 0, &t_default)) return rc;
     Tune t;
-    t.wpb = best_w;
-    t.bps = best_b;
-    t.us_per_voxel = best_ms * 1e3 / (double)V;
+    t.wpb = t_default <= best_ms ? 0 : best_w;
+    t.bps = t_default <= best_ms ? 0 : best_b;
+    t.us_per_voxel = std::min<double>(t_default, best_ms) * 1e3 / (double)V;
     ctx->tune[k] = t;
-    if (out) { out->warps_per_block = t.wpb; out->us_per_voxel = t.us_per_voxel; out->blocks_per_sm = t.bps; }
+    if (out) { out->warps_per_block = best_w; out->us_per_voxel = t.us_per_voxel; out->blocks_per_sm = best_b; }
     return DECAES_OK;
 }
 
@@ -1755,7 +1767,7 @@ std::vector<Chunk> srv_launch_tick(decaes_server *S) {
             (is_mixed(ch[q].r->mo) ? any_mixed : any_plain) = true;
         }
         k.kern = dk::batch_kernel(legacy, any_plain, any_mixed);
-        k.wpb = tuned_wpb(ctx, ch[k.first].r->mo);
+        k.wpb = launch_wpb(ctx, ch[k.first].r->mo, k.kern, k.smem_stride);
         ok = launch_shape(ctx, k.kern, k.smem_stride, &k.wpb, &k.grid, &k.smem, tuned_bps(ctx, ch[k.first].r->mo)) == DECAES_OK;
         scr_doubles = std::max(scr_doubles, k.scr_stride * k.grid * k.wpb);
     }

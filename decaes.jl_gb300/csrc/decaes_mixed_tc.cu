@@ -10,6 +10,6 @@
 
 namespace dk {
 
-__global__ void __launch_bounds__(128) k_voxels_mixed_tc(const __grid_constant__ Params P) { voxels_body(P); }
+__global__ void __launch_bounds__(512) k_voxels_mixed_tc(const __grid_constant__ Params P) { voxels_body(P); }
 
 }  // namespace dk

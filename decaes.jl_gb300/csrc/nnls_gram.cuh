@@ -99,6 +99,31 @@ __device__ __forceinline__ double widen(float f) {
     return __longlong_as_double((long long)(sgn | mag));
 }
 
+// Tile of the factorization: the lower triangle of the matrix still to be
+// factored with the right-hand side as a row below it, in one run of shared
+// memory.  Rows and columns count from the end -- rho = k - r for matrix row r,
+// 0 for the right-hand side; gamma = k - c -- and element (rho, gamma), rho <=
+// gamma, has number gamma (gamma + 1) / 2 + rho.  So the trailing elements of
+// every step, of any k, are the first numbers.  gamma of a number is the count
+// of triangular numbers up to it: those before its block of 32 numbers, and a
+// bit mask of those in the block (one constant load, one population count).
+struct TileBlocks {
+    unsigned mask[66];  // triangular numbers in block s, and how many (of 1, 3, 6, ...) come before it
+    int below[66];
+    constexpr TileBlocks() : mask(), below() {
+        for (int s = 0; s < 66; ++s)
+            for (int g = 1; g * (g + 1) / 2 < 32 * s + 32; ++g)
+                if (g * (g + 1) / 2 < 32 * s) below[s] = g;
+                else mask[s] |= 1u << (g * (g + 1) / 2 - 32 * s);
+    }
+};
+static __constant__ const TileBlocks kTile;
+// element e = 32 s + lane (also entry (rho, gamma) of the packed Gram matrix)
+__device__ __forceinline__ void tile_element(int s, int e, unsigned lanes_le, int &rho, int &gamma) {
+    gamma = kTile.below[s] + __popc(kTile.mask[s] & lanes_le);
+    rho = e - tri(gamma);
+}
+
 // b'b.
 static __device__ void gram_bb(GramWS &g, int m, const ShD b) {
     const int lane = threadIdx.x & 31;
@@ -164,25 +189,29 @@ static __device__ __noinline__ void gram_build_f32(GramWS &g, const Sh<float> As
         g.f[j] = s0 + s1;
     }
     gram_bb(g, m, b);
-    const int npairs = tri(n);
+    // 32 entries at a time from the last: As reaches into G from below, and an
+    // entry overwrites only columns that none before it reads
+    const unsigned lanes_le = (2u << lane) - 1u;
     #pragma unroll 1
-    for (int p = lane; p < npairs; p += 32) {
-        int j = (int)((sqrtf(8.0f * (float)p + 1.0f) - 1.0f) * 0.5f);
-        while (tri(j) > p) --j;
-        while (tri(j + 1) <= p) ++j;
-        const int i = p - tri(j);
-        const Sh<float> ai = As + i * lda, aj = As + j * lda;
+    for (int b0 = (tri(n) - 1) >> 5; b0 >= 0; --b0) {
+        const int p = 32 * b0 + lane;
         double s0 = 0.0, s1 = 0.0;
-        int r = 0;
-        #pragma unroll 1
-        for (; r + 1 < m; r += 2) {
-            s0 = fma(widen(ai[r]), widen(aj[r]), s0);
-            s1 = fma(widen(ai[r + 1]), widen(aj[r + 1]), s1);
+        if (p < tri(n)) {
+            int i, j;
+            tile_element(b0, p, lanes_le, i, j);
+            const Sh<float> ai = As + i * lda, aj = As + j * lda;
+            int r = 0;
+            #pragma unroll 1
+            for (; r + 1 < m; r += 2) {
+                s0 = fma(widen(ai[r]), widen(aj[r]), s0);
+                s1 = fma(widen(ai[r + 1]), widen(aj[r + 1]), s1);
+            }
+            if (r < m) s0 = fma(widen(ai[r]), widen(aj[r]), s0);
         }
-        if (r < m) s0 = fma(widen(ai[r]), widen(aj[r]), s0);
-        g.G[p] = s0 + s1;
+        __syncwarp();
+        if (p < tri(n)) g.G[p] = s0 + s1;
+        __syncwarp();
     }
-    __syncwarp();
 }
 
 // G copied from a precomputed packed Gram matrix in global memory.
@@ -192,31 +221,6 @@ static __device__ __noinline__ void gram_load(GramWS &g, const double *Gg, int n
 #pragma unroll 4
     for (int q = lane; q < np; q += 32) g.G[q] = __ldg(Gg + q);
     __syncwarp();
-}
-
-// Tile of the factorization: the lower triangle of the matrix still to be
-// factored with the right-hand side as a row below it, in one run of shared
-// memory.  Rows and columns count from the end -- rho = k - r for matrix row r,
-// 0 for the right-hand side; gamma = k - c -- and element (rho, gamma), rho <=
-// gamma, has number gamma (gamma + 1) / 2 + rho.  So the trailing elements of
-// every step, of any k, are the first numbers.  gamma of a number is the count
-// of triangular numbers up to it: those before its block of 32 numbers, and a
-// bit mask of those in the block (one constant load, one population count).
-struct TileBlocks {
-    unsigned mask[66];  // triangular numbers in block s, and how many (of 1, 3, 6, ...) come before it
-    int below[66];
-    constexpr TileBlocks() : mask(), below() {
-        for (int s = 0; s < 66; ++s)
-            for (int g = 1; g * (g + 1) / 2 < 32 * s + 32; ++g)
-                if (g * (g + 1) / 2 < 32 * s) below[s] = g;
-                else mask[s] |= 1u << (g * (g + 1) / 2 - 32 * s);
-    }
-};
-static __constant__ const TileBlocks kTile;
-// element e = 32 s + lane
-__device__ __forceinline__ void tile_element(int s, int e, unsigned lanes_le, int &rho, int &gamma) {
-    gamma = kTile.below[s] + __popc(kTile.mask[s] & lanes_le);
-    rho = e - tri(gamma);
 }
 
 // LDL' factorization of H_PP = G_PP + mu2 I from scratch (right-looking) for k

@@ -1184,7 +1184,7 @@ static __device__ void warp_basis(Warp &w, double alpha, double *out /* m x n, g
 }
 
 // Mixed method: the same curves with the recursion in FP32 (coefficients in
-// FP64, rounded once), states in the Gram and factor regions, curves written
+// FP64, rounded once), states in the factor and Gram regions, curves written
 // as FP32 to the warp's global scratch, then staged in w.As32 and widened
 // (exactly, on the integer pipes) into w.A.  The basis of the voxel is these
 // FP32 values, for the Gram matrix and the fitted curve alike, and no FP32 <->
@@ -1192,7 +1192,7 @@ static __device__ void warp_basis(Warp &w, double alpha, double *out /* m x n, g
 static __device__ void warp_basis_f32(Warp &w, double alpha) {
     const Params &P = *w.P;
     const int m = P.m, n = P.n, lanes = P.epg_lanes_f32, lane = w.lane;
-    const Sh<float> S = w.g.G.as<float>();  // 3*m*lanes floats, lane-contiguous
+    const Sh<float> S = w.g.L.as<float>();  // 3*m*lanes floats, lane-contiguous, over the factor and Gram regions
     float *Af = reinterpret_cast<float *>(w.scr + warp_scratch_f32_offset(m, n, P.K));
     #pragma unroll 1
     for (int j0 = 0; j0 < n; j0 += lanes) {

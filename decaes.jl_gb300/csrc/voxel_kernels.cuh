@@ -19,17 +19,19 @@ static __device__ void warp_setup(Warp &w, const Params &P, ShD p, double *scr) 
         // normal-equation workspace (see warp_smem_doubles_mixed)
         const int m = P.m;
         w.data = p; p += m;
-        w.s.x = p; p += n;
-        w.s.w = p; p += n;
         w.xout = p; p += n;
-        w.g.G = p; p += (int)mixed_r1_doubles(m, n);
         w.g.L = p; p += w.g.nL = (int)mixed_r2_doubles(m, n, P.reg == 2);
+        w.g.G = p; p += (int)mixed_r1_doubles(m, n);  // follows L: the staged basis extends into it
         w.g.f = p; p += n;
         w.g.y = p; p += n;
         w.g.dd = p; p += n;
         w.g.dinv = p; p += n;
         w.g.xp = p; p += n;
         p += 8;
+        // the solver reads the duals only until it factors, and writes x when it
+        // is done: both share its scratch
+        w.s.w = w.g.dd;
+        w.s.x = w.g.xp;
         const ShI ip = p.as<int>();
         w.s.idx = ip;
         w.g.P = ip + n;

@@ -215,10 +215,12 @@ void decaes_batch_destroy(decaes_batch *batch);
 /* Autotuner: times the voxel kernel on a synthetic slab of the given shape
  * and method for a set of launch shapes -- 1, 2 and 4 warps (voxels in
  * flight) per block, each with as many resident blocks per SM as fit and with
- * one and two fewer -- keeps the fastest for that (nTE, nT2, nRefAngles, Reg,
- * precision, control angle) in the context, and reports it.  Later calls,
- * batches and server ticks on the context use the tuned shape; batches also
- * use the measured cost to order their queue. */
+ * one and two fewer -- and for the shape an untuned call takes (the block size
+ * that keeps the most warps resident), and keeps the fastest for that (nTE,
+ * nT2, nRefAngles, Reg, precision, control angle) in the context.  It reports
+ * the fastest of the former and the cost of the shape kept.  Later calls,
+ * batches and server ticks on the context use the kept shape; batches also use
+ * the measured cost to order their queue. */
 typedef struct {
     int32_t warps_per_block;
     double us_per_voxel;       /* device time per above-threshold voxel, whole GPU */
