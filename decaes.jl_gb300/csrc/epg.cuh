@@ -12,7 +12,8 @@
 //
 // State storage (S_: a pointer to T, or a view indexed like one) is strided so a warp can keep one curve per lane in shared
 // memory with lane-contiguous layout: F(k) = S[(k-1)*st], Fbar(k) =
-// S[(ETL+k-1)*st], Z(k) = S[(2*ETL+k-1)*st].
+// S[(ns+k-1)*st], Z(k) = S[(2*ns+k-1)*st], ns = epg_states(ETL): the echo train
+// uses the first half of its ETL states and one more.
 #pragma once
 #include <cmath>
 
@@ -61,10 +62,40 @@ DX_HD Dual absd(Dual a) { return signbit(a.v) ? -a : a; }
 DX_HD double absd(double a) { return fabs(a); }
 DX_HD double zero_of(double) { return 0.0; }
 DX_HD Dual zero_of(Dual) { return Dual{0.0, 0.0}; }
-// single-precision recursion of the mixed method
-DX_HD float fmad(float a, float b, float c) { return fmaf(a, b, c); }
-DX_HD float absd(float a) { return fabsf(a); }
-DX_HD float zero_of(float) { return 0.0f; }
+#ifdef __CUDACC__
+// The mixed method's single-precision recursion, two curves at a time: a pair of
+// floats in the packed FP32 instructions (each half rounded as the scalar
+// operation rounds it).
+struct F2 {
+    unsigned long long v;
+};
+__device__ __forceinline__ F2 mk2(float x, float y) {
+    return F2{(unsigned long long)__float_as_uint(y) << 32 | __float_as_uint(x)};
+}
+__device__ __forceinline__ float2 split(F2 a) {
+    return make_float2(__uint_as_float((unsigned)a.v), __uint_as_float((unsigned)(a.v >> 32)));
+}
+__device__ __forceinline__ F2 operator+(F2 a, F2 b) {
+    F2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ F2 fmad(F2 a, F2 b, F2 c) {
+    F2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+    return r;
+}
+// A product as fma(a, b, -0), the same rounding, with a -0 the assembler does not
+// know: it contracts mul.rn.f32x2 into a following add.rn.f32x2, -fmad=false or
+// not, which the scalar recursion does not do.
+static __constant__ unsigned long long kNegZero2 = 0x8000000080000000ull;
+__device__ __forceinline__ F2 operator*(F2 a, F2 b) { return fmad(a, b, F2{kNegZero2}); }
+__device__ __forceinline__ F2 operator-(F2 a) { return F2{a.v ^ 0x8000000080000000ull}; }
+__device__ __forceinline__ F2 operator-(F2 a, F2 b) { return a + -b; }
+__device__ __forceinline__ F2 operator/(F2 a, int two) { return a * mk2(1.0f / two, 1.0f / two); }  // two = 2: exact
+__device__ __forceinline__ F2 absd(F2 a) { return F2{a.v & 0x7fffffff7fffffffull}; }
+__device__ __forceinline__ F2 zero_of(F2) { return F2{0ull}; }
+#endif
 
 // sind: the degree reduction of Base.sind with a double-double radian
 // argument (sin(h + l) = sin h + l cos h to first order).
@@ -91,25 +122,36 @@ DX_HD double sind(double x) {
     return sin_dd(rx - copysign(360.0, rx));
 }
 
-// Coefficients of the constant-flip recursion, src/EPGdecaycurve.jl:955-962.
+// Coefficients of the constant-flip recursion, src/EPGdecaycurve.jl:955-962:
+// the part that all T2 times share, and one T2 time's.
 template <class T>
 struct FlatCoef {
     T a, b, c, d, cp, m0;
 };
-DX_HD FlatCoef<double> flat_coef(double alpha_deg, double TE, double T2, double T1) {
-    double al = alpha_deg * kD2R;
-    double E1 = pm_exp(-(TE / 2) / T1), E2 = pm_exp(-(TE / 2) / T2);
-    double sa, ca;
-    pm_sincos(al, &sa, &ca);
-    double E22h = (E2 * E2) / 2, E1E2 = E1 * E2, E11 = E1 * E1;
+struct FlatAngle {
+    double sa, ca, E1, m0;
+};
+DX_HD FlatAngle flat_angle(double alpha_deg, double TE, double T1) {
+    FlatAngle g;
+    g.E1 = pm_exp(-(TE / 2) / T1);
+    pm_sincos(alpha_deg * kD2R, &g.sa, &g.ca);
+    g.m0 = sind(alpha_deg / 2);
+    return g;
+}
+DX_HD FlatCoef<double> flat_coef(const FlatAngle &g, double TE, double T2) {
+    double E2 = pm_exp(-(TE / 2) / T2);
+    double E22h = (E2 * E2) / 2, E1E2 = g.E1 * E2, E11 = g.E1 * g.E1;
     FlatCoef<double> k;
     k.a = E22h;
-    k.b = E22h * ca;
-    k.c = E1E2 * sa;
-    k.d = E11 * ca;
+    k.b = E22h * g.ca;
+    k.c = E1E2 * g.sa;
+    k.d = E11 * g.ca;
     k.cp = -k.c / 2;
-    k.m0 = sind(alpha_deg / 2);
+    k.m0 = g.m0;
     return k;
+}
+DX_HD FlatCoef<double> flat_coef(double alpha_deg, double TE, double T2, double T1) {
+    return flat_coef(flat_angle(alpha_deg, TE, T1), TE, T2);
 }
 DX_HD FlatCoef<Dual> flat_coef_dual(double alpha_deg, double TE, double T2, double T1) {
     Dual al{alpha_deg * kD2R, kD2R};
@@ -128,11 +170,14 @@ DX_HD FlatCoef<Dual> flat_coef_dual(double alpha_deg, double TE, double T2, doub
     return k;
 }
 
-// Coefficients rounded to single precision (mixed method; the coefficients
-// themselves are evaluated in FP64).
-DX_HD FlatCoef<float> to_f32(const FlatCoef<double> &k) {
-    return FlatCoef<float>{(float)k.a, (float)k.b, (float)k.c, (float)k.d, (float)k.cp, (float)k.m0};
+#ifdef __CUDACC__
+// Two curves' coefficients rounded to single precision (mixed method; the
+// coefficients themselves are evaluated in FP64).
+__device__ __forceinline__ F2 to_f2(double x, double y) { return mk2((float)x, (float)y); }
+__device__ __forceinline__ FlatCoef<F2> to_f2(const FlatCoef<double> &k, const FlatCoef<double> &l) {
+    return FlatCoef<F2>{to_f2(k.a, l.a), to_f2(k.b, l.b), to_f2(k.c, l.c), to_f2(k.d, l.d), to_f2(k.cp, l.cp), to_f2(k.m0, l.m0)};
 }
+#endif
 
 // One state of the constant-flip step: outputs (F of state k+1, Fbar of
 // state k-1, Z of state k) from (F, Fbar, Z) of state k.
@@ -144,15 +189,18 @@ DX_HD void flat_state(const FlatCoef<T> &q, T F, T Fb, T Z, T &oF, T &oFb, T &oZ
     oZ = fmad(q.cp, S, q.d * Z);
 }
 
-// epg_decay_curve! for the constant-flip kernel: impulse response, then
-// dc[i] = |m0 * dc[i]|.  S holds 3*ETL strided values (st apart).
+// epg_decay_curve! for the constant-flip kernel: the impulse response's echoes
+// times m0, as absolute values, to dc.  S holds 3*epg_states(ETL) strided values
+// (st apart).
+DX_HD int epg_states(int ETL) { return (ETL + 1) / 2 + 1; }
 template <class T, class S_, class O>
-DX_HD void epg_flat_inplace(int ETL, const FlatCoef<T> &q, S_ S, int st, O *dc, int dst) {
+DX_HD void epg_flat_inplace(int ETL, const FlatCoef<T> &q, S_ S, int st, O dc, int dst) {
+    const int ns = epg_states(ETL);
 #define EF(k) S[((k)-1) * st]
-#define EFb(k) S[(ETL + (k)-1) * st]
-#define EZ(k) S[(2 * ETL + (k)-1) * st]
+#define EFb(k) S[(ns + (k)-1) * st]
+#define EZ(k) S[(2 * ns + (k)-1) * st]
     const T z0 = zero_of(q.a);
-    dc[0] = q.a - q.b;
+    dc[0] = absd(q.m0 * (q.a - q.b));
     EF(1) = q.a - q.b; EFb(1) = z0; EZ(1) = q.cp;
     EF(2) = q.a + q.b; EFb(2) = z0; EZ(2) = z0;
     for (int i = 2; i <= ETL - 1; ++i) {
@@ -165,7 +213,7 @@ DX_HD void epg_flat_inplace(int ETL, const FlatCoef<T> &q, S_ S, int st, O *dc, 
             flat_state(q, Fk, Fbk, Zk, oF, oFb, oZ);
             if (k == 1) {
                 EF(1) = oFb;
-                dc[(i - 1) * dst] = oFb;
+                dc[(i - 1) * dst] = absd(q.m0 * oFb);
             } else {
                 EFb(k - 1) = oFb;
             }
@@ -181,9 +229,8 @@ DX_HD void epg_flat_inplace(int ETL, const FlatCoef<T> &q, S_ S, int st, O *dc, 
     {
         T F = EF(1), Fb = EFb(1), Z = EZ(1);
         T C = F + Fb, S2 = F - Fb;
-        dc[(ETL - 1) * dst] = fmad(-q.c, Z, fmad(q.a, C, (-q.b) * S2));
+        dc[(ETL - 1) * dst] = absd(q.m0 * fmad(-q.c, Z, fmad(q.a, C, (-q.b) * S2)));
     }
-    for (int i = 0; i < ETL; ++i) dc[i * dst] = absd(q.m0 * dc[i * dst]);
 #undef EF
 #undef EFb
 #undef EZ
@@ -240,17 +287,19 @@ DX_HD VecCoef<Dual> vec_coef_dual(double alpha_deg, double TE, double T2, double
     return k;
 }
 
-DX_HD VecCoef<float> to_f32(const VecCoef<double> &k) {
-    VecCoef<float> o;
-    for (int c = 0; c < 3; ++c) { o.F[c] = (float)k.F[c]; o.Fb[c] = (float)k.Fb[c]; o.Z[c] = (float)k.Z[c]; }
-    o.a1 = (float)k.a1; o.b1 = (float)k.b1; o.c1 = (float)k.c1; o.m0 = (float)k.m0;
+#ifdef __CUDACC__
+__device__ __forceinline__ VecCoef<F2> to_f2(const VecCoef<double> &k, const VecCoef<double> &l) {
+    VecCoef<F2> o;
+    for (int c = 0; c < 3; ++c) { o.F[c] = to_f2(k.F[c], l.F[c]); o.Fb[c] = to_f2(k.Fb[c], l.Fb[c]); o.Z[c] = to_f2(k.Z[c], l.Z[c]); }
+    o.a1 = to_f2(k.a1, l.a1); o.b1 = to_f2(k.b1, l.b1); o.c1 = to_f2(k.c1, l.c1); o.m0 = to_f2(k.m0, l.m0);
     return o;
 }
+#endif
 
 // epg_decay_curve! for EPGOptions (DualVector_Split_Dynamic), in place.
-// S holds 3*ETL strided values: state k's (x,y,z) at S[(3(k-1)+c)*st].
+// S holds 3*epg_states(ETL) strided values: state k's (x,y,z) at S[(3(k-1)+c)*st].
 template <class T, class S_, class O>
-DX_HD void epg_vec_inplace(int ETL, const VecCoef<T> &q, S_ S, int st, O *dc, int dst) {
+DX_HD void epg_vec_inplace(int ETL, const VecCoef<T> &q, S_ S, int st, O dc, int dst) {
 #define SX(k, c) S[(3 * ((k)-1) + (c)) * st]
     const T z0 = zero_of(q.m0);
     T M0x = q.b1 * q.m0, M0z = ((-q.c1) * q.m0) / 2;

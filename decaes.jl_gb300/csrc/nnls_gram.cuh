@@ -98,6 +98,12 @@ __device__ __forceinline__ double widen(float f) {
                                           : ((unsigned long long)(e + (1023 - 127)) << 52) | ((unsigned long long)(u & 0x7fffffu) << 29);
     return __longlong_as_double((long long)(sgn | mag));
 }
+// The same for a value with its sign bit clear (an EPG curve is an absolute
+// value), in half the instructions.
+__device__ __forceinline__ double widen_abs(float f) {
+    const unsigned u = __float_as_uint(f);
+    return __hiloint2double(u < 0x800000u ? 0 : (int)((u >> 3) + 0x38000000u), u < 0x800000u ? 0 : (int)(u << 29));
+}
 
 // Tile of the factorization: the lower triangle of the matrix still to be
 // factored with the right-hand side as a row below it, in one run of shared
@@ -149,7 +155,6 @@ static __device__ __noinline__ void gram_rhs_t(GramWS &g, const double *AT, int 
         if (i < m) s0 = fma(__ldg(AT + (long)i * n + j), b[i], s0);
         g.f[j] = s0 + s1;
     }
-    gram_bb(g, m, b);
     __syncwarp();
 }
 
@@ -164,7 +169,6 @@ static __device__ __noinline__ void gram_rhs_f32(GramWS &g, const float *F, int 
         const float2 v = __ldg(reinterpret_cast<const float2 *>(F) + j);
         g.f[j] = (widen(v.x) + widen(v.y)) * scale;
     }
-    gram_bb(g, m, b);
     __syncwarp();
 }
 
@@ -182,13 +186,12 @@ static __device__ __noinline__ void gram_build_f32(GramWS &g, const Sh<float> As
         int i = 0;
         #pragma unroll 1
         for (; i + 1 < m; i += 2) {
-            s0 = fma(widen(aj[i]), b[i], s0);
-            s1 = fma(widen(aj[i + 1]), b[i + 1], s1);
+            s0 = fma(widen_abs(aj[i]), b[i], s0);
+            s1 = fma(widen_abs(aj[i + 1]), b[i + 1], s1);
         }
-        if (i < m) s0 = fma(widen(aj[i]), b[i], s0);
+        if (i < m) s0 = fma(widen_abs(aj[i]), b[i], s0);
         g.f[j] = s0 + s1;
     }
-    gram_bb(g, m, b);
     // 32 entries at a time from the last: As reaches into G from below, and an
     // entry overwrites only columns that none before it reads
     const unsigned lanes_le = (2u << lane) - 1u;
@@ -203,10 +206,10 @@ static __device__ __noinline__ void gram_build_f32(GramWS &g, const Sh<float> As
             int r = 0;
             #pragma unroll 1
             for (; r + 1 < m; r += 2) {
-                s0 = fma(widen(ai[r]), widen(aj[r]), s0);
-                s1 = fma(widen(ai[r + 1]), widen(aj[r + 1]), s1);
+                s0 = fma(widen_abs(ai[r]), widen_abs(aj[r]), s0);
+                s1 = fma(widen_abs(ai[r + 1]), widen_abs(aj[r + 1]), s1);
             }
-            if (r < m) s0 = fma(widen(ai[r]), widen(aj[r]), s0);
+            if (r < m) s0 = fma(widen_abs(ai[r]), widen_abs(aj[r]), s0);
         }
         __syncwarp();
         if (p < tri(n)) g.G[p] = s0 + s1;
@@ -404,11 +407,12 @@ static __device__ __noinline__ bool gram_append(const GramWS g, int k, int t, do
     if (!gt_nonneg_bits(delta, kGramDepTol * htt)) return false;
     const double yt = g.f[t] - ly;
     if (!pos_bits(yt)) return false;
+    const double rd = fast_rcp(delta);
     const ShD Lk = g.L + tri(k - 1);
     if (r0 < k) Lk[r0] = w0;
     if (r1 < k) Lk[r1] = w1;
     if (lane == 0) {
-        g.dinv[k] = fast_rcp(delta);
+        g.dinv[k] = rd;
         g.y[k] = yt;
         g.P[k] = t;
     }

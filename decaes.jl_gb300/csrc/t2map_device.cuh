@@ -1163,7 +1163,7 @@ static __device__ double flip_angle_search(Warp &w, double mx, long slot) {
 static __device__ void warp_basis(Warp &w, double alpha, double *out /* m x n, global */) {
     const Params &P = *w.P;
     const int m = P.m, n = P.n, lanes = P.epg_lanes, lane = w.lane;
-    const ShD S = w.s.C;  // 3*m*lanes doubles, lane-contiguous, over the C, b and zz regions
+    const ShD S = w.s.C;  // 3*epg_states(m)*lanes doubles, lane-contiguous, over the C, b and zz regions
     #pragma unroll 1
     for (int j0 = 0; j0 < n; j0 += lanes) {
         int j = j0 + lane;
@@ -1183,28 +1183,49 @@ static __device__ void warp_basis(Warp &w, double alpha, double *out /* m x n, g
     __syncwarp();
 }
 
+// A pair of curves' echoes to row-major FP32 storage (columns j and j + 1 side by side).
+struct PairOut {
+    float *p;
+    bool both;
+    struct Ref {
+        float *p;
+        bool both;
+        __device__ __forceinline__ void operator=(dx::F2 v) const {
+            const float2 x = dx::split(v);
+            p[0] = x.x;
+            if (both) p[1] = x.y;
+        }
+    };
+    __device__ __forceinline__ Ref operator[](int i) const { return Ref{p + i, both}; }
+};
 // Mixed method: the same curves with the recursion in FP32 (coefficients in
-// FP64, rounded once), states in the factor and Gram regions, curves written
-// as FP32 to the warp's global scratch, then staged in w.As32 and widened
-// (exactly, on the integer pipes) into w.A.  The basis of the voxel is these
-// FP32 values, for the Gram matrix and the fitted curve alike, and no FP32 <->
-// FP64 conversion occupies the FP64 pipe.
+// FP64, rounded once), two T2 columns per lane in the packed FP32 instructions,
+// states in the factor and Gram regions, curves written as FP32 rows to the
+// warp's global scratch, then staged in w.As32 and widened (exactly, on the
+// integer pipes) into w.A.  The basis of the voxel is these FP32 values, for the
+// Gram matrix and the fitted curve alike, and no FP32 <-> FP64 conversion
+// occupies the FP64 pipe.  (One column per lane, 22 lanes at 48 echoes and 40
+// columns, took two rounds of scalar instructions; with the packed ones 240x240x4 chi2
+// 91.6 -> 86.8 ms, 240x240x1 L-curve 54.6 -> 53.1 ms.)
 static __device__ void warp_basis_f32(Warp &w, double alpha) {
     const Params &P = *w.P;
     const int m = P.m, n = P.n, lanes = P.epg_lanes_f32, lane = w.lane;
-    const Sh<float> S = w.g.L.as<float>();  // 3*m*lanes floats, lane-contiguous, over the factor and Gram regions
+    const Sh<dx::F2> S = w.g.L.as<dx::F2>();  // 3*epg_states(m)*lanes pairs, lane-contiguous
     float *Af = reinterpret_cast<float *>(w.scr + warp_scratch_f32_offset(m, n, P.K));
     #pragma unroll 1
-    for (int j0 = 0; j0 < n; j0 += lanes) {
-        int j = j0 + lane;
+    for (int j0 = 0; j0 < n; j0 += 2 * lanes) {
+        const int j = j0 + 2 * lane, j1 = j + 1 < n ? j + 1 : j;
         if (lane < lanes && j < n) {
-            const Sh<float> Sl = S + lane;
+            const Sh<dx::F2> Sl = S + lane;
+            const PairOut out{Af + j, j + 1 < n};
             if (P.beta180) {
-                dx::FlatCoef<float> q = dx::to_f32(dx::flat_coef(alpha, P.TE, P.t2[j], P.T1));
-                dx::epg_flat_inplace(m, q, Sl, lanes, Af + (long)j * m, 1);
+                const dx::FlatAngle g = dx::flat_angle(alpha, P.TE, P.T1);
+                const dx::FlatCoef<dx::F2> q = dx::to_f2(dx::flat_coef(g, P.TE, P.t2[j]), dx::flat_coef(g, P.TE, P.t2[j1]));
+                dx::epg_flat_inplace(m, q, Sl, lanes, out, n);
             } else {
-                dx::VecCoef<float> q = dx::to_f32(dx::vec_coef(alpha, P.TE, P.t2[j], P.T1, P.beta));
-                dx::epg_vec_inplace(m, q, Sl, lanes, Af + (long)j * m, 1);
+                const dx::VecCoef<dx::F2> q = dx::to_f2(dx::vec_coef(alpha, P.TE, P.t2[j], P.T1, P.beta),
+                                                        dx::vec_coef(alpha, P.TE, P.t2[j1], P.T1, P.beta));
+                dx::epg_vec_inplace(m, q, Sl, lanes, out, n);
             }
         }
         __syncwarp();
@@ -1212,12 +1233,14 @@ static __device__ void warp_basis_f32(Warp &w, double alpha) {
     __threadfence_block();
     __syncwarp();
     #pragma unroll 1
-    for (long q = lane; q < (long)m * n; q += 32) {
-        const int i = (int)(q % m), j = (int)(q / m);
-        const float v = Af[q];
-        w.A[q] = widen(v);
-        w.As32[i + w.ldA * j] = v;
-    }
+    for (int j = lane; j < n; j += 32)
+        #pragma unroll 4
+        for (int i = 0; i < m; ++i) w.As32[i + w.ldA * j] = Af[(long)i * n + j];
+    __syncwarp();
+    #pragma unroll 1
+    for (int j = 0; j < n; ++j)
+        #pragma unroll 1
+        for (int i = lane; i < m; i += 32) w.A[i + (long)m * j] = widen_abs(w.As32[i + w.ldA * j]);
     __threadfence_block();
     __syncwarp();
 }
@@ -1251,6 +1274,7 @@ static __device__ void process_voxel(Warp &w, long v, long slot = 0) {
 
     double alpha;
     w.g.lastk = 0;  // warm starts never cross voxels (results independent of scheduling)
+    if (use_mixed(w)) gram_bb(w.g, m, w.data);
     if (P.angle_mode == 1) {
         alpha = P.fixed_angle;
         w.A = const_cast<double *>(P.basis_fixed);

@@ -39,7 +39,7 @@ struct Params {
     int legacy;         // legacy algorithms: spline surrogate search, chi2 doubling search
     const double *Gs;   // packed Gram matrices A_k'A_k of the grid bases (K x n(n+1)/2), or of the fixed basis
     const double *AsT;  // the grid (or fixed) bases transposed, K x m x n (row-major per basis)
-    int epg_lanes_f32;  // lanes of the FP32 EPG (states in the Gram and factor regions)
+    int epg_lanes_f32;  // lanes of the FP32 EPG, two columns each (states in the factor and Gram regions)
     long smem_stride;   // doubles of shared memory per warp (several warps per block)
     // the voxel-list positions of a k_voxels_mixed_tc launch: [tq0, min(tq1, *nvox))
     long tq0, tq1;
@@ -95,12 +95,12 @@ __host__ __device__ inline long warp_smem_doubles_mixed(int m, int n, bool gcv) 
     long ints = 2L * n;  // idx, P
     return d + (ints * 4 + 7) / 8;
 }
-// Lanes of the FP64 method's EPG basis (one T2 column per lane, 3m states
-// each).  The states use the contiguous C, b and zz regions of the workspace
-// (lda * (n + 2) doubles, free while the voxel's basis is built), which hold
-// at least one lane's states for every n >= 1 because lda >= m + n.
+// Lanes of the FP64 method's EPG basis (one T2 column per lane, 3 * ((m + 1) / 2
+// + 1) states each).  The states use the contiguous C, b and zz regions of the
+// workspace (lda * (n + 2) doubles, free while the voxel's basis is built), which
+// hold at least one lane's states for every n >= 1 because lda >= m + n.
 __host__ __device__ inline int fp64_epg_lanes(int m, int n, int lda) {
-    long l = ((long)lda * (n + 2)) / (3L * m);
+    long l = ((long)lda * (n + 2)) / (3L * ((m + 1) / 2 + 1));
     return (int)(l < 1 ? 1 : (l > 32 ? 32 : l));
 }
 // Global scratch of one warp worker (doubles).
