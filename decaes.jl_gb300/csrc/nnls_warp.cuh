@@ -199,9 +199,11 @@ static __device__ double warp_cah(const NnlsWS &s, int ip, int jp, int m) {
     if (xnorm == 0) return -1.0;
     double beta = copysign(xnorm, alpha);
     alpha = alpha + beta;
-    const double rbeta = 1.0 / beta;
-    double tau = mdiv(alpha, beta, rbeta);
-    const double ralpha = 1.0 / alpha;
+    // 1 / alpha, alpha / beta and 1 / beta in one division, a lane each (a
+    // division is ~10 FP64 warp instructions whatever its active lanes)
+    const double qd = (lane == 1 ? alpha : 1.0) / (lane == 0 ? alpha : beta);
+    const double ralpha = bcast(qd, 0), rbeta = bcast(qd, 2);
+    double tau = bcast(qd, 1);
     // quotients A[i,jp]/alpha, staged in zz (free between solves of the main loop)
     part = 0.0;
     for (int i = ip + 1 + lane; i <= m; i += 32) {
@@ -289,9 +291,35 @@ static __device__ void warp_compute_dual(const NnlsWS &s, int n, int j1, int m1)
 }
 
 // zz[1:n] = b[1:n]; solve_triangular_system!(zz, A, n), src/NNLS.jl:506-523.
-// Lanes over rows; the column sweep is sequential as in the reference.
+// Lanes over rows; the column sweep is sequential as in the reference.  Up to
+// 64 rows stay on their lanes (two each), so a step of the chain passes through
+// one shuffle instead of shared memory and two warp barriers.
 static __device__ void warp_solve_tri(const NnlsWS &s, int n) {
     const int lane = threadIdx.x & 31;
+    if (n <= 64) {
+        double z0 = lane < n ? s.b[lane] : 0.0, z1 = lane + 32 < n ? s.b[lane + 32] : 0.0;
+        #pragma unroll 1
+        for (int j = n; j > 32; --j) {
+            const int pj = s.idx[j - 1] - 1;
+            const ShD a = s.C + pj * s.lda;
+            const double zj = mdiv(bcast(z1, j - 33), a[j - 1], s.rdiag[pj]), zi = -zj;
+            z0 = fma(a[lane], zi, z0);
+            if (lane < j - 33) z1 = fma(a[lane + 32], zi, z1);
+            if (lane == j - 33) z1 = zj;
+        }
+        #pragma unroll 1
+        for (int j = min(n, 32); j >= 1; --j) {
+            const int pj = s.idx[j - 1] - 1;
+            const ShD a = s.C + pj * s.lda;
+            const double zj = mdiv(bcast(z0, j - 1), a[j - 1], s.rdiag[pj]), zi = -zj;
+            if (lane < j - 1) z0 = fma(a[lane], zi, z0);
+            if (lane == j - 1) z0 = zj;
+        }
+        if (lane < n) s.zz[lane] = z0;
+        if (lane + 32 < n) s.zz[lane + 32] = z1;
+        __syncwarp();
+        return;
+    }
     for (int i = lane; i < n; i += 32) s.zz[i] = s.b[i];
     __syncwarp();
     for (int j = n; j >= 1; --j) {
@@ -446,24 +474,23 @@ static __device__ NnlsResult warp_nnls(const NnlsWS &s, int M, int n, int m0, bo
                         const ShD ci = s.C + (s.idx[i - 1] - 1) * s.lda;
                         double a = ci[i - 2], bb = ci[i - 1];
                         double sg = jl_hypot(a, bb);
-                        double cc = a / sg, ss = bb / sg;
+                        // both rotation coefficients and 1 / sg in one division, a lane each
+                        const double qd = (lane == 0 ? a : (lane == 1 ? bb : 1.0)) / sg;
+                        const double cc = bcast(qd, 0), ss = bcast(qd, 1);
                         __syncwarp();
                         const int pi = s.idx[i - 1] - 1;
-                        for (int pj = lane; pj < n; pj += 32) {
+                        // the other columns, and b as column n
+                        for (int pj = lane; pj <= n; pj += 32) {
                             if (pj == pi) continue;
-                            const ShD cj = s.C + pj * s.lda;
+                            const ShD cj = pj < n ? s.C + pj * s.lda : s.b;
                             double p = cj[i - 2], r = cj[i - 1];
                             cj[i - 2] = fma(cc, p, __dmul_rn(ss, r));
                             cj[i - 1] = fma(-ss, p, __dmul_rn(cc, r));
                         }
-                        const double rsg = 1.0 / sg;
-                        if (lane == 0) {
+                        if (lane == 2) {
                             ci[i - 2] = sg;
                             ci[i - 1] = 0.0;
-                            s.rdiag[s.idx[i - 1] - 1] = rsg;
-                            double p = s.b[i - 2], r = s.b[i - 1];
-                            s.b[i - 2] = fma(cc, p, __dmul_rn(ss, r));
-                            s.b[i - 1] = fma(-ss, p, __dmul_rn(cc, r));
+                            s.rdiag[pi] = qd;
                         }
                         __syncwarp();
                     }
