@@ -19,6 +19,12 @@
 //     lanes-over-rows with butterfly reductions (reassociated sums, like the
 //     reference's @simd loops).
 // Every loop is bounded; the NNLS iteration cap is the reference's 3n.
+//
+// Only the sequential column loops are unrolled (8 rows: their loads overlap);
+// the lane-strided ones run one to three times and stay rolled, or the solver
+// would be 107 KB of code waiting for instruction fetch instead of 65: 32x32x4
+// voxels x 32 echoes, chi2, 18.5 -> 17.4 ms (17.7 with 2 rows, 17.4 with 4),
+// 120x120x1 x 48 echoes, L-curve, 128.2 -> 125.2 ms (128.6, 126.4).
 #pragma once
 #include <cuda_runtime.h>
 #include <math_constants.h>
@@ -138,6 +144,7 @@ struct NnlsWS {
 __device__ __forceinline__ int warp_active_cols(const NnlsWS &s, int n, int jfirst) {
     const int lane = threadIdx.x & 31;
     int base = 0;
+    #pragma unroll 1
     for (int c = 0; c < n; c += 32) {
         int p = c + lane;
         bool z = p < n && s.posof[p] >= jfirst;
@@ -194,6 +201,7 @@ static __device__ double warp_cah(const NnlsWS &s, int ip, int jp, int m) {
     const ShD col = s.C + (s.idx[jp - 1] - 1) * s.lda;  // pivot column (0-based rows)
     double alpha = col[ip - 1];
     double part = 0.0;
+    #pragma unroll 1
     for (int i = ip + lane; i <= m; i += 32) part = fma(col[i - 1], col[i - 1], part);
     double xnorm = sqrt(wsum(part));
     if (xnorm == 0) return -1.0;
@@ -206,6 +214,7 @@ static __device__ double warp_cah(const NnlsWS &s, int ip, int jp, int m) {
     double tau = bcast(qd, 1);
     // quotients A[i,jp]/alpha, staged in zz (free between solves of the main loop)
     part = 0.0;
+    #pragma unroll 1
     for (int i = ip + 1 + lane; i <= m; i += 32) {
         double qi = mdiv(col[i - 1], alpha, ralpha);
         s.zz[i - 1] = qi;
@@ -222,6 +231,7 @@ static __device__ double warp_cah(const NnlsWS &s, int ip, int jp, int m) {
     if (good) {
         if (ip < m) {
             __syncwarp();
+            #pragma unroll 1
             for (int i = ip + 1 + lane; i <= m; i += 32) {
                 double qi = s.zz[i - 1];
                 col[i - 1] = qi;
@@ -252,16 +262,19 @@ static __device__ void warp_ahd(const NnlsWS &s, int n, double tau, int j1, int 
     if (j1 >= m1) return;
     const ShD u = s.C + (s.idx[j1 - 1] - 1) * s.lda;  // u[j1-1] is the diagonal; treated as 1
     const int nz = warp_active_cols(s, n, j1 + 1);
+    #pragma unroll 1
     for (int r0 = 0; r0 < nz; r0 += 32) {
         int r = r0 + lane;
         if (r < nz) {
             const int p = s.zl[r];
             const ShD a = s.C + p * s.lda;
             double sm = fma(a[j1 - 1], 1.0, 0.0);
+            #pragma unroll 8
             for (int i = j1 + 1; i <= m1; ++i) sm = fma(a[i - 1], u[i - 1], sm);
             sm *= -tau;
             double wj = 0.0;
             a[j1 - 1] = a[j1 - 1] + sm;
+            #pragma unroll 8
             for (int i = j1 + 1; i <= m1; ++i) {
                 double v = fma(sm, u[i - 1], a[i - 1]);
                 wj = fma(v, s.b[i - 1], wj);
@@ -277,12 +290,14 @@ static __device__ void warp_ahd(const NnlsWS &s, int n, double tau, int j1, int 
 static __device__ void warp_compute_dual(const NnlsWS &s, int n, int j1, int m1) {
     const int lane = threadIdx.x & 31;
     const int nz = warp_active_cols(s, n, j1);
+    #pragma unroll 1
     for (int r0 = 0; r0 < nz; r0 += 32) {
         int r = r0 + lane;
         if (r < nz) {
             const int p = s.zl[r];
             const ShD a = s.C + p * s.lda;
             double sm = 0.0;
+            #pragma unroll 8
             for (int i = j1; i <= m1; ++i) sm = fma(a[i - 1], s.b[i - 1], sm);
             s.w[s.posof[p] - 1] = sm;
         }
@@ -320,12 +335,15 @@ static __device__ void warp_solve_tri(const NnlsWS &s, int n) {
         __syncwarp();
         return;
     }
+    #pragma unroll 1
     for (int i = lane; i < n; i += 32) s.zz[i] = s.b[i];
     __syncwarp();
+    #pragma unroll 1
     for (int j = n; j >= 1; --j) {
         const int pj = s.idx[j - 1] - 1;
         const ShD a = s.C + pj * s.lda;
         double zi = -mdiv(s.zz[j - 1], a[j - 1], s.rdiag[pj]);
+        #pragma unroll 1
         for (int i = 1 + lane; i <= j - 1; i += 32) s.zz[i - 1] = fma(a[i - 1], zi, s.zz[i - 1]);
         __syncwarp();
         if (lane == 0) s.zz[j - 1] = -zi;
@@ -336,9 +354,11 @@ static __device__ void warp_solve_tri(const NnlsWS &s, int n) {
 // Transposed solve (U' z = x) on the first n logical columns, src/NNLS.jl:524-537.
 static __device__ void warp_solve_tri_t(const NnlsWS &s, ShD z, int n) {
     const int lane = threadIdx.x & 31;
+    #pragma unroll 1
     for (int j = 1; j <= n; ++j) {
         const ShD a = s.C + (s.idx[j - 1] - 1) * s.lda;
         double part = 0.0;
+        #pragma unroll 1
         for (int l = 1 + lane; l <= j - 1; l += 32) part = fma(-a[l - 1], z[l - 1], part);
         double z1 = z[j - 1] + wsum(part);
         z1 /= a[j - 1];
@@ -355,6 +375,7 @@ __device__ __forceinline__ void warp_largest_dual(const NnlsWS &s, int n, int j1
     const int lane = threadIdx.x & 31;
     long long km = 0;
     int jm = 0;
+    #pragma unroll 1
     for (int j = j1 + lane; j <= n; j += 32) {
         long long k = __double_as_longlong(s.w[j - 1]);
         if (k > 0 && k <= 0x7ff0000000000000LL && k > km) { km = k; jm = j; }
@@ -383,10 +404,12 @@ static __device__ NnlsResult warp_nnls(const NnlsWS &s, int M, int n, int m0, bo
     int m = tikh ? m0 : M;
     int nsetp = 0, iter = 0, mode = 0;
     bool terminated = false;
+    #pragma unroll 1
     for (;;) {
         if (nsetp >= n || (!tikh && nsetp >= m)) break;
         int jmax = nsetp;
         double tau = 0.0;
+        #pragma unroll 1
         for (;;) {
             double wmax;
             warp_largest_dual(s, n, nsetp + 1, wmax, jmax);
@@ -423,6 +446,7 @@ static __device__ NnlsResult warp_nnls(const NnlsWS &s, int M, int n, int m0, bo
         if (nsetp < n) warp_ahd(s, n, tau, nsetp, m);
         {
             const ShD pc = s.C + (s.idx[nsetp - 1] - 1) * s.lda;
+            #pragma unroll 1
             for (int i = nsetp + 1 + lane; i <= m; i += 32) pc[i - 1] = 0.0;
         }
         __syncwarp();
@@ -430,6 +454,7 @@ static __device__ NnlsResult warp_nnls(const NnlsWS &s, int M, int n, int m0, bo
         __syncwarp();
         warp_solve_tri(s, nsetp);
         bool dual_flag = false;
+        #pragma unroll 1
         for (;;) {
             iter += 1;
             if (iter > max_iter) { mode = 1; terminated = true; break; }
@@ -440,6 +465,7 @@ static __device__ NnlsResult warp_nnls(const NnlsWS &s, int M, int n, int m0, bo
                 long long a_key = okey(2.0);
                 double a_loc = 2.0;
                 int i_loc = 0;
+                #pragma unroll 1
                 for (int i = 1 + lane; i <= nsetp; i += 32) {
                     double zi = s.zz[i - 1];
                     if (!isnan_bits(zi) && okey(zi) <= 0) {
@@ -460,16 +486,19 @@ static __device__ NnlsResult warp_nnls(const NnlsWS &s, int M, int n, int m0, bo
             }
             if (alpha == 2.0) break;
             dual_flag = true;
+            #pragma unroll 1
             for (int i = 1 + lane; i <= nsetp; i += 32) {
                 int ix = s.idx[i - 1] - 1;
                 s.x[ix] = fma(alpha, s.zz[i - 1] - s.x[ix], s.x[ix]);
             }
             __syncwarp();
             // move coefficient imv (and any infeasible ones) from set P to set Z
+            #pragma unroll 1
             for (int guard = 0; guard <= n; ++guard) {
                 if (lane == 0) s.x[s.idx[imv - 1] - 1] = 0.0;
                 __syncwarp();
                 if (imv != nsetp) {
+                    #pragma unroll 1
                     for (int i = imv + 1; i <= nsetp; ++i) {
                         const ShD ci = s.C + (s.idx[i - 1] - 1) * s.lda;
                         double a = ci[i - 2], bb = ci[i - 1];
@@ -480,6 +509,7 @@ static __device__ NnlsResult warp_nnls(const NnlsWS &s, int M, int n, int m0, bo
                         __syncwarp();
                         const int pi = s.idx[i - 1] - 1;
                         // the other columns, and b as column n
+                        #pragma unroll 1
                         for (int pj = lane; pj <= n; pj += 32) {
                             if (pj == pi) continue;
                             const ShD cj = pj < n ? s.C + pj * s.lda : s.b;
@@ -497,6 +527,7 @@ static __device__ NnlsResult warp_nnls(const NnlsWS &s, int M, int n, int m0, bo
                     // move logical column imv to position nsetp (idx rotation; no data moves)
                     if (lane == 0) {
                         int t = s.idx[imv - 1];
+                        #pragma unroll 1
                         for (int j = imv; j <= nsetp - 1; ++j) {
                             s.idx[j - 1] = s.idx[j];
                             s.posof[s.idx[j - 1] - 1] = j;
@@ -509,6 +540,7 @@ static __device__ NnlsResult warp_nnls(const NnlsWS &s, int M, int n, int m0, bo
                 nsetp -= 1;
                 // first remaining infeasible coefficient, if any
                 int bad = 0;
+                #pragma unroll 1
                 for (int ib = 1; ib <= nsetp; ib += 32) {
                     int i = ib + lane;
                     bool neg = (i <= nsetp) && (s.x[s.idx[i - 1] - 1] <= 0);
@@ -522,6 +554,7 @@ static __device__ NnlsResult warp_nnls(const NnlsWS &s, int M, int n, int m0, bo
         }
         if (terminated) break;
         if (dual_flag) warp_compute_dual(s, n, nsetp + 1, m);
+        #pragma unroll 1
         for (int i = 1 + lane; i <= nsetp; i += 32) s.x[s.idx[i - 1] - 1] = s.zz[i - 1];
         __syncwarp();
     }
@@ -529,8 +562,10 @@ static __device__ NnlsResult warp_nnls(const NnlsWS &s, int M, int n, int m0, bo
     const int rows = tikh ? M : m;
     double part = 0.0;
     if (nsetp < rows) {
+        #pragma unroll 1
         for (int i = nsetp + 1 + lane; i <= rows; i += 32) part = fma(s.b[i - 1], s.b[i - 1], part);
     } else {
+        #pragma unroll 1
         for (int j = lane; j < n; j += 32) s.w[j] = 0.0;
     }
     __syncwarp();
@@ -552,12 +587,16 @@ static __device__ __noinline__ NnlsResult warp_lsq(const NnlsWS s, const double 
     const int lane = threadIdx.x & 31;
     const int M = tikh ? m + n : m;
     // C[:, j] = A[:, j] (coalesced), padded rows zeroed
+    #pragma unroll 1
     for (int j = 0; j < n; ++j) {
         const double *aj = A + (size_t)j * m;
         const ShD cj = s.C + j * s.lda;
+        #pragma unroll 1
         for (int i = lane; i < M; i += 32) cj[i] = (i < m) ? aj[i] : 0.0;
     }
+    #pragma unroll 1
     for (int i = lane; i < M; i += 32) s.b[i] = (i < m) ? data[i] : 0.0;
+    #pragma unroll 1
     for (int j = lane; j < n; j += 32) {
         s.x[j] = 0.0;
         s.idx[j] = j + 1;
@@ -567,21 +606,26 @@ static __device__ __noinline__ NnlsResult warp_lsq(const NnlsWS s, const double 
     __syncwarp();
     const ShD an = s.C + (n - 1) * s.lda;
     double part = 0.0;
+    #pragma unroll 1
     for (int i = lane; i < m; i += 32) part = __dadd_rn(part, __dmul_rn(an[i], an[i]));
     double den = wsum(part);
     if (tikh) den = __dadd_rn(den, __dmul_rn(mu, mu));
     const double rden = 1.0 / den;
     part = 0.0;
+    #pragma unroll 1
     for (int i = lane; i < m; i += 32) part = __dadd_rn(part, __dmul_rn(mdiv(an[i], den, rden), data[i]));
     double xj = wsum(part);
+    #pragma unroll 1
     for (int i = lane; i < m; i += 32) s.zz[i] = __dsub_rn(data[i], __dmul_rn(an[i], xj));
     __syncwarp();
     bool pos = false;
+    #pragma unroll 1
     for (int jb = 0; jb < n - 1; jb += 32) {
         int j = jb + lane;
         if (j < n - 1) {
             const ShD cj = s.C + j * s.lda;
             double wj = 0.0;
+            #pragma unroll 8
             for (int i = 0; i < m; ++i) wj = __dadd_rn(wj, __dmul_rn(cj[i], s.zz[i]));
             s.w[j] = wj;
             pos |= !(wj <= 0);
@@ -597,6 +641,7 @@ static __device__ __noinline__ NnlsResult warp_lsq(const NnlsWS s, const double 
 static __device__ double warp_seminorm_sq(const NnlsWS &s, int nsetp) {
     const int lane = threadIdx.x & 31;
     double part = 0.0;
+    #pragma unroll 1
     for (int i = lane; i < nsetp; i += 32) {
         double v = s.x[s.idx[i] - 1];
         part = __dadd_rn(part, __dmul_rn(v, v));
