@@ -467,6 +467,7 @@ static __device__ __noinline__ void gram_svdvals(GramWS g, const ShD W, int m, i
     for (int q = lane; q < np; q += 32) W[q] = g.G[q];
     __syncwarp();
     const ShD d = g.dd, e = g.dinv, u = g.y, qv = g.xp;
+    const unsigned lanes_le = (2u << lane) - 1u;
     // 1. tridiagonalization (Householder from the left and right, column k)
 #pragma unroll 1
     for (int k = 0; k + 2 < n; ++k) {
@@ -511,13 +512,16 @@ static __device__ __noinline__ void gram_svdvals(GramWS g, const ShD W, int m, i
 #pragma unroll 1
         for (int r = k + 1 + lane; r < n; r += 32) qv[r] = fma(-K, u[r], qv[r]);
         __syncwarp();
-        // W22 -= u q' + q u' (lower triangle, row r owned by its lane)
-#pragma unroll 1
-        for (int r = k + 1 + lane; r < n; r += 32) {
-            const int br = tri(r);
-            const double ur = u[r], qr = qv[r];
-#pragma unroll 1
-            for (int c = k + 1; c <= r; ++c) W[br + c] = fma(-ur, qv[c], fma(-qr, u[c], W[br + c]));
+        // W22 -= u q' + q u' (lower triangle), lanes over its entries
+        const int t = n - k - 1;
+        #pragma unroll 1
+        for (int s = 0, e = lane; e < tri(t); ++s, e += 32) {
+            int c, r;
+            tile_element(s, e, lanes_le, c, r);
+            c += k + 1;
+            r += k + 1;
+            const int w = tri(r) + c;
+            W[w] = fma(-u[r], qv[c], fma(-qv[r], u[c], W[w]));
         }
         __syncwarp();
     }
@@ -545,22 +549,17 @@ static __device__ __noinline__ void gram_svdvals(GramWS g, const ShD W, int m, i
     // Sturm count: eigenvalues of the tridiagonal matrix below x
     auto count_below = [&](double x) {
         double p2 = 1.0, p1 = d[0] - x;
-        bool neg = p1 <= 0;  // a zero takes the sign opposite to its predecessor (p_0 = +1)
+        bool neg = sturm_neg(p1, false);  // (p_0 = +1)
         int c = neg;
-#pragma unroll 1
+#pragma unroll 2
         for (int j = 1; j < n; ++j) {
-            double p = fma(d[j] - x, p1, -e2[j - 1] * p2);
-            bool pneg = p < 0 || (p == 0 && !neg);
+            const double p = fma(d[j] - x, p1, -e2[j - 1] * p2);
+            const bool pneg = sturm_neg(p, neg);
             c += (pneg != neg);
             neg = pneg;
             p2 = p1;
             p1 = p;
-            const int ex = ((__double2hiint(p1) >> 20) & 0x7ff) - 1023;
-            if (p1 != 0 && (ex > 400 || ex < -400)) {
-                const double sc = __hiloint2double((1023 - ex) << 20, 0);
-                p1 *= sc;
-                p2 *= sc;
-            }
+            sturm_rescale(p1, p2);
         }
         return c;
     };

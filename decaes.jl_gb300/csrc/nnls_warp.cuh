@@ -85,6 +85,23 @@ __device__ __forceinline__ bool gt_nonneg_bits(double d, double t) {
     const long long b = __double_as_longlong(d);
     return b > __double_as_longlong(t) && b <= 0x7ff0000000000000LL && !isnan_bits(t);
 }
+// Steps of a Sturm sequence on the integer pipes (an FP64 comparison holds the
+// FP64 pipe like any other FP64 instruction): whether p counts as negative (a
+// zero takes the sign opposite to its predecessor's), and the rescaling of the
+// last two terms by a power of two once the exponent leaves +-400.
+__device__ __forceinline__ bool sturm_neg(double p, bool neg) {
+    const unsigned long long u = (unsigned long long)__double_as_longlong(p);
+    if ((u << 1) == 0) return !neg;
+    return u > 0x8000000000000000ull && u <= 0xfff0000000000000ull;  // p < 0, NaN excluded
+}
+__device__ __forceinline__ void sturm_rescale(double &p1, double &p2) {
+    const int hi = __double2hiint(p1), f = hi & 0x7ff00000;
+    if ((unsigned)(f - (623 << 20)) > (800u << 20) && (((unsigned)hi << 1) | (unsigned)__double2loint(p1)) != 0u) {
+        const double sc = __hiloint2double((2046 << 20) - f, 0);
+        p1 *= sc;
+        p2 *= sc;
+    }
+}
 // wsum of two values at once: the first butterfly step exchanges a and b
 // between the warp halves, so both sums take five additions instead of ten;
 // each sum is added in wsum's order, so the results are wsum's bit for bit.

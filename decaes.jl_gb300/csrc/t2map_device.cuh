@@ -810,23 +810,19 @@ static __device__ void warp_svdvals(Warp &w, double *gam) {
     const double tau0 = 1e-14 * bnd, atol = 1e-15 * bnd;
     // Sturm count: eigenvalues of the tridiagonal below x (zero diagonal)
     auto count_below = [&](double x) {
-        double p2 = 1.0, p1 = 0.0 - x;
-        bool neg = p1 <= 0;  // a zero takes the sign opposite to its predecessor (p_0 = +1)
+        const double mx = 0.0 - x;
+        double p2 = 1.0, p1 = mx;
+        bool neg = sturm_neg(p1, false);  // (p_0 = +1)
         int cnt = neg;
-        #pragma unroll 1
+        #pragma unroll 2
         for (int j = 1; j < N; ++j) {
-            double p = fma(0.0 - x, p1, -o2[j - 1] * p2);
-            bool pneg = p < 0 || (p == 0 && !neg);
+            const double p = fma(mx, p1, -o2[j - 1] * p2);
+            const bool pneg = sturm_neg(p, neg);
             cnt += (pneg != neg);
             neg = pneg;
             p2 = p1;
             p1 = p;
-            const int ex = ((__double2hiint(p1) >> 20) & 0x7ff) - 1023;
-            if (p1 != 0 && (ex > 400 || ex < -400)) {
-                const double sc = __hiloint2double((1023 - ex) << 20, 0);
-                p1 *= sc;
-                p2 *= sc;
-            }
+            sturm_rescale(p1, p2);
         }
         return cnt;
     };
