@@ -566,24 +566,9 @@ static __device__ __noinline__ void gram_svdvals(GramWS g, const ShD W, int m, i
     const int nz = count_below(tau);  // eigenvalues below tau: left at zero
     const int kk = m < n ? m : n;
     const int nres = n - nz;  // resolved eigenvalues (the largest)
-#pragma unroll 1
-    for (int base = 0; base < nres; base += 32) {
-        const int t = base + lane;       // t-th largest eigenvalue
-        const bool mine = t < nres;
-        const int idx = n - 1 - t;       // its index in ascending order
-        double a = tau, b = bnd;
-        bool done = !mine;
-#pragma unroll 1
-        for (int it = 0; it < 80 && __any_sync(FULL, !done); ++it) {
-            const double mid = 0.5 * (a + b);
-            const int c = count_below(mid);
-            if (!done) {
-                if (c > idx) b = mid; else a = mid;
-                done = (b - a) <= fmax(atol, 4.0 * 2.220446049250313e-16 * b);
-            }
-        }
-        if (mine && t < kk) gam[t] = sqrt(0.5 * (a + b));
-    }
+    warp_bisect(count_below, n, nres, tau, bnd, atol, u, qv, [&](int t, double a, double b) {
+        if (t < kk) gam[t] = sqrt(0.5 * (a + b));
+    });
 #pragma unroll 1
     for (int t = nres + lane; t < kk; t += 32) gam[t] = 0.0;
     __syncwarp();

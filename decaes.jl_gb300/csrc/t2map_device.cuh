@@ -827,24 +827,9 @@ static __device__ void warp_svdvals(Warp &w, double *gam) {
         return cnt;
     };
     const int nres = N - count_below(tau0);  // singular values >= tau0 (the rest are left at zero)
-    #pragma unroll 1
-    for (int base = 0; base < nres; base += 32) {
-        const int t = base + lane;  // t-th largest singular value
-        const bool mine = t < nres;
-        const int idx = N - 1 - t;  // its index among the eigenvalues in ascending order
-        double a = tau0, b = bnd;
-        bool done = !mine;
-        #pragma unroll 1
-        for (int it = 0; it < 80 && __any_sync(FULL, !done); ++it) {
-            const double mid = 0.5 * (a + b);
-            const int cnt = count_below(mid);
-            if (!done) {
-                if (cnt > idx) b = mid; else a = mid;
-                done = (b - a) <= fmax(atol, 4.0 * 2.220446049250313e-16 * b);
-            }
-        }
-        if (mine && t < c) gam[t] = 0.5 * (a + b);
-    }
+    warp_bisect(count_below, N, nres, tau0, bnd, atol, dv, ev, [&](int t, double a, double b) {
+        if (t < c) gam[t] = 0.5 * (a + b);
+    });
     #pragma unroll 1
     for (int t = nres + lane; t < c; t += 32) gam[t] = 0.0;
     __syncwarp();
