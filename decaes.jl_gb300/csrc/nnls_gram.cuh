@@ -139,21 +139,24 @@ static __device__ void gram_bb(GramWS &g, int m, const ShD b) {
     g.bb = wsum(part);
 }
 
-// f = A'b from a row-major (transposed, m x n) basis in global memory: lanes
-// over columns, coalesced over each row.
+// f = A'b from a row-major (transposed, m x n) basis in global memory: a lane
+// per column and row parity (the even and the odd rows have sums of their own,
+// added at the end), so 40 columns take 3 rounds of 24 rows instead of 2 of 48;
+// four loads are in flight.
 static __device__ __noinline__ void gram_rhs_t(GramWS &g, const double *AT, int m, int n, const ShD b) {
-    const int lane = threadIdx.x & 31;
+    const int lane = threadIdx.x & 31, par = lane & 1;
     #pragma unroll 1
-    for (int j = lane; j < n; j += 32) {
-        double s0 = 0.0, s1 = 0.0;
-        int i = 0;
-        #pragma unroll 1
-        for (; i + 1 < m; i += 2) {
-            s0 = fma(__ldg(AT + (long)i * n + j), b[i], s0);
-            s1 = fma(__ldg(AT + (long)(i + 1) * n + j), b[i + 1], s1);
+    for (int t = lane; t - lane < 2 * n; t += 32) {
+        const int j = t >> 1;
+        double s = 0.0;
+        if (j < n) {
+            const double *a = AT + j;
+            #pragma unroll 4
+            for (int i = par; i < m; i += 2) s = fma(__ldg(a + (long)i * n), b[i], s);
         }
-        if (i < m) s0 = fma(__ldg(AT + (long)i * n + j), b[i], s0);
-        g.f[j] = s0 + s1;
+        __syncwarp();
+        s = s + __shfl_xor_sync(FULL, s, 1);
+        if (par == 0 && j < n) g.f[j] = s;
     }
     __syncwarp();
 }
@@ -217,12 +220,19 @@ static __device__ __noinline__ void gram_build_f32(GramWS &g, const Sh<float> As
     }
 }
 
-// G copied from a precomputed packed Gram matrix in global memory.
+// Starts the copy of G from a precomputed packed Gram matrix in global memory;
+// gram_load_wait before it is read.  Asynchronous copies need no registers, so
+// all of them are in flight at once, behind the right-hand side's products.
 static __device__ __noinline__ void gram_load(GramWS &g, const double *Gg, int n) {
     const int lane = threadIdx.x & 31;
     const int np = tri(n);
 #pragma unroll 4
-    for (int q = lane; q < np; q += 32) g.G[q] = __ldg(Gg + q);
+    for (int q = lane; q < np; q += 32)
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((unsigned)__cvta_generic_to_shared(&g.G[q])), "l"(Gg + q)
+                     : "memory");
+}
+__device__ __forceinline__ void gram_load_wait() {
+    asm volatile("cp.async.wait_all;" ::: "memory");
     __syncwarp();
 }
 

@@ -915,6 +915,7 @@ static __device__ void fa_update(Search &S, int I) {
         else
 #endif
             gram_rhs_t(w.g, P.AsT + (long)(I - 1) * m * n, m, n, w.data);
+        gram_load_wait();
         r = gram_nnls(w.g, w.s.x, w.s.w, w.s.idx, n, 0.0, 3 * n, &w.g.lastk);
     } else {
         r = warp_lsq(w.s, A, m, n, w.data, false, 0.0);
@@ -923,26 +924,32 @@ static __device__ void fa_update(Search &S, int I) {
     double ell = __dmul_rn(r.rnorm, r.rnorm);
     double part = 0;
     #pragma unroll 1
-    for (int i0 = 0; i0 < (kLegacyKernel && P.legacy ? 0 : m); i0 += 32) {  // legacy: loss! only, src/splines.jl:1043-1046
-        int i = i0 + lane;
-        double ax = 0, dax = 0;
+    for (int i0 = lane; i0 - lane < (kLegacyKernel && P.legacy ? 0 : m); i0 += 64) {  // legacy: loss! only, src/splines.jl:1043-1046
+        const bool h0 = i0 < m, h1 = i0 + 32 < m;  // two rows a lane: their loads of a column are in flight together
+        double ax0 = 0, dax0 = 0, ax1 = 0, dax1 = 0;
         // the columns with x_j > 0 in increasing order, from one ballot per 32
         // columns instead of a comparison per column
         #pragma unroll 1
         for (int j0 = 0; j0 < n; j0 += 32) {
             unsigned msk = __ballot_sync(FULL, j0 + lane < n && pos_bits(w.s.x[j0 + lane]));
-            if (i < m) {
-                #pragma unroll 1
-                while (msk) {
-                    const int j = j0 + __ffs(msk) - 1;
-                    msk &= msk - 1;
-                    const double xj = w.s.x[j];
-                    ax = fma(xj, __ldg(A + i + (long)j * m), ax);
-                    dax = fma(xj, __ldg(dA + i + (long)j * m), dax);
+            #pragma unroll 1
+            while (msk) {
+                const int j = j0 + __ffs(msk) - 1;
+                msk &= msk - 1;
+                const double xj = w.s.x[j];
+                const double *Aj = A + i0 + (long)j * m, *dAj = dA + i0 + (long)j * m;
+                const double a0 = h0 ? __ldg(Aj) : 0.0, d0 = h0 ? __ldg(dAj) : 0.0;
+                const double a1 = h1 ? __ldg(Aj + 32) : 0.0, d1 = h1 ? __ldg(dAj + 32) : 0.0;
+                ax0 = fma(xj, a0, ax0);
+                dax0 = fma(xj, d0, dax0);
+                if (h1) {
+                    ax1 = fma(xj, a1, ax1);
+                    dax1 = fma(xj, d1, dax1);
                 }
             }
         }
-        if (i < m) part = fma(dax, ax - w.data[i], part);
+        if (h0) part = fma(dax0, ax0 - w.data[i0], part);
+        if (h1) part = fma(dax1, ax1 - w.data[i0 + 32], part);
     }
     double dt = wsum(part);
     if (lane == 0) {
@@ -1276,6 +1283,7 @@ static __device__ void process_voxel(Warp &w, long v, long slot = 0) {
         if (P.angle_mode == 1) {
             gram_load(w.g, P.Gs, n);
             gram_rhs_t(w.g, P.AsT, m, n, w.data);
+            gram_load_wait();
         } else {
             gram_build_f32(w.g, w.As32, w.ldA, m, n, w.data);
         }
