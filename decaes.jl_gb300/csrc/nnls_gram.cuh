@@ -56,22 +56,6 @@ struct GramWS {
     double bb;     // b'b
 };
 
-// Warp-wide maximum of the bit patterns of non-negative doubles (0: no entry)
-// and the smallest index j that holds it; warp_bitsmin likewise the minimum.
-// Three integer warp reductions instead of a butterfly's fifteen shuffles.
-__device__ __forceinline__ unsigned long long warp_bitsmax(unsigned long long v, int &j) {
-    const unsigned hi = (unsigned)(v >> 32), lo = (unsigned)v;
-    const unsigned mh = __reduce_max_sync(FULL, hi), ml = __reduce_max_sync(FULL, hi == mh ? lo : 0u);
-    j = (int)__reduce_min_sync(FULL, hi == mh && lo == ml ? (unsigned)j : 0xffffffffu);
-    return (unsigned long long)mh << 32 | ml;
-}
-__device__ __forceinline__ unsigned long long warp_bitsmin(unsigned long long v, int &j) {
-    const unsigned hi = (unsigned)(v >> 32), lo = (unsigned)v;
-    const unsigned mh = __reduce_min_sync(FULL, hi), ml = __reduce_min_sync(FULL, hi == mh ? lo : 0xffffffffu);
-    j = (int)__reduce_min_sync(FULL, hi == mh && lo == ml ? (unsigned)j : 0xffffffffu);
-    return (unsigned long long)mh << 32 | ml;
-}
-
 // 1/d for normal d: the hardware's approximate FP64 reciprocal (rcp.approx,
 // relative error below 2^-20) refined by one cubic Newton step
 // r(1 + e + e^2), e = 1 - d r, whose error e^3 is below FP64 rounding.

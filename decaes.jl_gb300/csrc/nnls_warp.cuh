@@ -76,6 +76,11 @@ __device__ __forceinline__ bool pos_bits(double d) {
     const long long b = __double_as_longlong(d);
     return b > 0 && b <= 0x7ff0000000000000LL;
 }
+// d <= 0 on the integer pipes (true for zeros, false for NaN).
+__device__ __forceinline__ bool nonpos_bits(double d) {
+    const long long b = __double_as_longlong(d);
+    return !isnan_bits(d) && (b <= 0);
+}
 // d > t for a threshold t with its sign bit clear (+0.0 or positive) or NaN,
 // on the integer pipes: such doubles order like their bit patterns; negative d
 // and NaN d give false, and so does every d against a NaN threshold, as the
@@ -85,6 +90,22 @@ __device__ __forceinline__ bool gt_nonneg_bits(double d, double t) {
     const long long b = __double_as_longlong(d);
     return b > __double_as_longlong(t) && b <= 0x7ff0000000000000LL && !isnan_bits(t);
 }
+// Warp-wide maximum of the bit patterns of non-negative doubles (0: no entry)
+// and the smallest index j that holds it; warp_bitsmin likewise the minimum.
+// Three integer warp reductions instead of a butterfly's fifteen shuffles.
+__device__ __forceinline__ unsigned long long warp_bitsmax(unsigned long long v, int &j) {
+    const unsigned hi = (unsigned)(v >> 32), lo = (unsigned)v;
+    const unsigned mh = __reduce_max_sync(FULL, hi), ml = __reduce_max_sync(FULL, hi == mh ? lo : 0u);
+    j = (int)__reduce_min_sync(FULL, hi == mh && lo == ml ? (unsigned)j : 0xffffffffu);
+    return (unsigned long long)mh << 32 | ml;
+}
+__device__ __forceinline__ unsigned long long warp_bitsmin(unsigned long long v, int &j) {
+    const unsigned hi = (unsigned)(v >> 32), lo = (unsigned)v;
+    const unsigned mh = __reduce_min_sync(FULL, hi), ml = __reduce_min_sync(FULL, hi == mh ? lo : 0xffffffffu);
+    j = (int)__reduce_min_sync(FULL, hi == mh && lo == ml ? (unsigned)j : 0xffffffffu);
+    return (unsigned long long)mh << 32 | ml;
+}
+
 // Steps of a Sturm sequence on the integer pipes (an FP64 comparison holds the
 // FP64 pipe like any other FP64 instruction): whether p counts as negative (a
 // zero takes the sign opposite to its predecessor's), and the rescaling of the
@@ -278,7 +299,7 @@ static __device__ double warp_cah(const NnlsWS &s, int ip, int jp, int m) {
     #pragma unroll 1
     for (int i = ip + lane; i <= m; i += 32) part = fma(col[i - 1], col[i - 1], part);
     double xnorm = sqrt(wsum(part));
-    if (xnorm == 0) return -1.0;
+    if ((__double_as_longlong(xnorm) << 1) == 0) return -1.0;  // xnorm == 0
     double beta = copysign(xnorm, alpha);
     alpha = alpha + beta;
     // 1 / alpha, alpha / beta and 1 / beta in one division, a lane each (a
@@ -298,9 +319,12 @@ static __device__ double warp_cah(const NnlsWS &s, int ip, int jp, int m) {
     sm *= -tau;
     double A1 = -beta;
     double b1 = s.b[ip - 1] + sm;
-    // b1 / A1 > 0: same nonzero sign and no underflow of the quotient
+    // b1 / A1 > 0: same nonzero sign and no underflow of the quotient (told by
+    // the bit patterns unless |b1| is 2^-899 of |A1| or a value is not normal)
+    const int hb = __double2hiint(b1), ha = __double2hiint(A1), eb = hb >> 20 & 0x7ff, ea = ha >> 20 & 0x7ff;
     bool good;
-    if (b1 != 0 && fabs(b1) > 0x1p-900 * fabs(A1)) good = (b1 > 0) == (A1 > 0);
+    if (eb > 0 && ea > 0 && eb < 0x7ff && ea < 0x7ff && eb > ea - 899) good = (hb ^ ha) >= 0;
+    else if (b1 != 0 && fabs(b1) > 0x1p-900 * fabs(A1)) good = (b1 > 0) == (A1 > 0);
     else good = b1 / A1 > 0;
     if (good) {
         if (ip < m) {
@@ -469,26 +493,21 @@ static __device__ void warp_solve_tri_t(const NnlsWS &s, ShD z, int n) {
     }
 }
 
-// Largest positive dual over logical positions j1..n (first maximum wins,
-// as the reference's `w[j] > wmax` scan from wmax = 0).  Positive doubles
-// order like their bit patterns, so the search runs on the integer pipes.
-__device__ __forceinline__ void warp_largest_dual(const NnlsWS &s, int n, int j1, double &wmax, int &jmax) {
+// Logical position j1..n of the largest positive dual (the first one, as the
+// reference's `w[j] > wmax` scan from wmax = 0), 0 when there is none.  Positive
+// doubles order like their bit patterns, so the search runs on the integer pipes.
+__device__ __forceinline__ int warp_largest_dual(const NnlsWS &s, int n, int j1) {
     const int lane = threadIdx.x & 31;
-    long long km = 0;
+    unsigned long long km = 0;
     int jm = 0;
     #pragma unroll 1
     for (int j = j1 + lane; j <= n; j += 32) {
-        long long k = __double_as_longlong(s.w[j - 1]);
-        if (k > 0 && k <= 0x7ff0000000000000LL && k > km) { km = k; jm = j; }
+        const double w = s.w[j - 1];
+        const unsigned long long k = (unsigned long long)__double_as_longlong(w);
+        if (pos_bits(w) && k > km) { km = k; jm = j; }
     }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        long long ok = __shfl_xor_sync(FULL, km, o);
-        int oj = __shfl_xor_sync(FULL, jm, o);
-        if (ok > km || (ok == km && oj != 0 && (jm == 0 || oj < jm))) { km = ok; jm = oj; }
-    }
-    wmax = __longlong_as_double(km);
-    jmax = jm;
+    warp_bitsmax(km, jm);
+    return jm;
 }
 
 struct NnlsResult {
@@ -512,15 +531,14 @@ static __device__ NnlsResult warp_nnls(const NnlsWS &s, int M, int n, int m0, bo
         double tau = 0.0;
         #pragma unroll 1
         for (;;) {
-            double wmax;
-            warp_largest_dual(s, n, nsetp + 1, wmax, jmax);
-            if (wmax <= 0) { terminated = true; break; }
+            jmax = warp_largest_dual(s, n, nsetp + 1);
+            if (jmax == 0) { terminated = true; break; }  // no positive dual
             if (tikh && !s.diag[s.idx[jmax - 1] - 1]) {
                 if (lane == 0) Aat(s, m + 1, jmax) = lam;
                 __syncwarp();
             }
             tau = warp_cah(s, nsetp + 1, jmax, tikh ? min(m + 1, M) : m);
-            if (tau >= 0) break;
+            if (!isnan_bits(tau) && __double_as_longlong(tau) >= 0) break;  // tau >= 0 (-1: refused)
             __syncwarp();
             if (lane == 0) {
                 s.w[jmax - 1] = 0.0;
@@ -562,6 +580,7 @@ static __device__ NnlsResult warp_nnls(const NnlsWS &s, int M, int n, int m0, bo
             // feasibility step, src/NNLS.jl:700-727 (first minimum wins)
             int imv = nsetp;
             double alpha = 2.0;
+            bool moved = false;
             {
                 long long a_key = okey(2.0);
                 double a_loc = 2.0;
@@ -576,16 +595,17 @@ static __device__ NnlsResult warp_nnls(const NnlsWS &s, int M, int n, int m0, bo
                         if (!isnan_bits(t) && a_key > tk) { a_key = tk; a_loc = t; i_loc = i; }
                     }
                 }
-#pragma unroll
-                for (int o = 16; o > 0; o >>= 1) {
+                moved = __any_sync(FULL, i_loc != 0);
+#pragma unroll 1
+                for (int o = moved ? 16 : 0; o > 0; o >>= 1) {
                     long long ok = __shfl_xor_sync(FULL, a_key, o);
                     double oa = __shfl_xor_sync(FULL, a_loc, o);
                     int oi = __shfl_xor_sync(FULL, i_loc, o);
                     if (oi != 0 && (i_loc == 0 || ok < a_key || (ok == a_key && oi < i_loc))) { a_key = ok; a_loc = oa; i_loc = oi; }
                 }
-                if (i_loc != 0) { imv = i_loc; alpha = a_loc; }
+                if (moved) { imv = i_loc; alpha = a_loc; }
             }
-            if (alpha == 2.0) break;
+            if (!moved) break;
             dual_flag = true;
             #pragma unroll 1
             for (int i = 1 + lane; i <= nsetp; i += 32) {
@@ -644,7 +664,7 @@ static __device__ NnlsResult warp_nnls(const NnlsWS &s, int M, int n, int m0, bo
                 #pragma unroll 1
                 for (int ib = 1; ib <= nsetp; ib += 32) {
                     int i = ib + lane;
-                    bool neg = (i <= nsetp) && (s.x[s.idx[i - 1] - 1] <= 0);
+                    bool neg = (i <= nsetp) && nonpos_bits(s.x[s.idx[i - 1] - 1]);
                     unsigned msk = __ballot_sync(FULL, neg);
                     if (msk) { bad = ib + __ffs(msk) - 1; break; }
                 }
@@ -729,7 +749,7 @@ static __device__ __noinline__ NnlsResult warp_lsq(const NnlsWS s, const double 
             #pragma unroll 8
             for (int i = 0; i < m; ++i) wj = __dadd_rn(wj, __dmul_rn(cj[i], s.zz[i]));
             s.w[j] = wj;
-            pos |= !(wj <= 0);
+            pos |= !nonpos_bits(wj);
         }
     }
     bool anypos = __any_sync(FULL, pos);
