@@ -205,19 +205,13 @@ static __device__ __noinline__ void gram_build_f32(GramWS &g, const Sh<float> As
 }
 
 // Starts the copy of G from a precomputed packed Gram matrix in global memory;
-// gram_load_wait before it is read.  Asynchronous copies need no registers, so
+// copy_async_wait before it is read.  Asynchronous copies need no registers, so
 // all of them are in flight at once, behind the right-hand side's products.
 static __device__ __noinline__ void gram_load(GramWS &g, const double *Gg, int n) {
     const int lane = threadIdx.x & 31;
     const int np = tri(n);
 #pragma unroll 4
-    for (int q = lane; q < np; q += 32)
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((unsigned)__cvta_generic_to_shared(&g.G[q])), "l"(Gg + q)
-                     : "memory");
-}
-__device__ __forceinline__ void gram_load_wait() {
-    asm volatile("cp.async.wait_all;" ::: "memory");
-    __syncwarp();
+    for (int q = lane; q < np; q += 32) copy_async(g.G + q, Gg + q);
 }
 
 // LDL' factorization of H_PP = G_PP + mu2 I from scratch (right-looking) for k

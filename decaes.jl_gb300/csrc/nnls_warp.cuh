@@ -216,6 +216,17 @@ static __device__ __forceinline__ void warp_bisect(Count &count_below, int N, in
     }
 }
 
+// An 8-byte copy from global to shared memory without a register in between;
+// copy_async_wait completes the warp's copies.
+__device__ __forceinline__ void copy_async(const ShD dst, const double *src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((unsigned)__cvta_generic_to_shared(dst.ptr())), "l"(src)
+                 : "memory");
+}
+__device__ __forceinline__ void copy_async_wait() {
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncwarp();
+}
+
 // Per-warp views of the NNLS workspace (shared memory).
 struct NnlsWS {
     ShD C;    // lda x n, physical columns
@@ -707,13 +718,16 @@ static __device__ __noinline__ NnlsResult warp_lsq(const NnlsWS s, const double 
                                             bool tikh, double mu) {
     const int lane = threadIdx.x & 31;
     const int M = tikh ? m + n : m;
-    // C[:, j] = A[:, j] (coalesced), padded rows zeroed
+    // C[:, j] = A[:, j] (coalesced, asynchronous: all copies in flight at once),
+    // padded rows zeroed
     #pragma unroll 1
     for (int j = 0; j < n; ++j) {
         const double *aj = A + (size_t)j * m;
         const ShD cj = s.C + j * s.lda;
         #pragma unroll 1
-        for (int i = lane; i < M; i += 32) cj[i] = (i < m) ? aj[i] : 0.0;
+        for (int i = lane; i < m; i += 32) copy_async(cj + i, aj + i);
+        #pragma unroll 1
+        for (int i = m + lane; i < M; i += 32) cj[i] = 0.0;
     }
     #pragma unroll 1
     for (int i = lane; i < M; i += 32) s.b[i] = (i < m) ? data[i] : 0.0;
@@ -724,7 +738,7 @@ static __device__ __noinline__ NnlsResult warp_lsq(const NnlsWS s, const double 
         s.posof[j] = j + 1;
         s.diag[j] = 0;
     }
-    __syncwarp();
+    copy_async_wait();
     const ShD an = s.C + (n - 1) * s.lda;
     double part = 0.0;
     #pragma unroll 1

@@ -915,7 +915,7 @@ static __device__ void fa_update(Search &S, int I) {
         else
 #endif
             gram_rhs_t(w.g, P.AsT + (long)(I - 1) * m * n, m, n, w.data);
-        gram_load_wait();
+        copy_async_wait();
         r = gram_nnls(w.g, w.s.x, w.s.w, w.s.idx, n, 0.0, 3 * n, &w.g.lastk);
     } else {
         r = warp_lsq(w.s, A, m, n, w.data, false, 0.0);
@@ -1283,7 +1283,7 @@ static __device__ void process_voxel(Warp &w, long v, long slot = 0) {
         if (P.angle_mode == 1) {
             gram_load(w.g, P.Gs, n);
             gram_rhs_t(w.g, P.AsT, m, n, w.data);
-            gram_load_wait();
+            copy_async_wait();
         } else {
             gram_build_f32(w.g, w.As32, w.ldA, m, n, w.data);
         }
