@@ -162,44 +162,97 @@ __global__ void k_batch_prefix(const int *counts, int nvol, int *offsets) {
     }
 }
 
-// Standalone T2partSEcorr (src/T2partSEcorr.jl:95-138): one thread per voxel.
+// T2partSEcorr's sums of one voxel, each in its own loop order; value(j) is the
+// distribution's j-th entry as FP64.
+template <class Value>
+__device__ __forceinline__ void t2part_voxel(Value value, int n, int sp0, int sp1, int mp0, int mp1, const double *logt2,
+                                             const double *weights, double (&o)[4]) {
+    double sd = 0, ssp = 0, smp = 0, dsp = 0, dmp = 0;
+    #pragma unroll 4
+    for (int j = 0; j < n; ++j) sd = __dadd_rn(sd, value(j));
+    #pragma unroll 4
+    for (int j = sp0; j <= sp1; ++j) {
+        const double d = value(j);
+        dsp = __dadd_rn(dsp, __dmul_rn(d, logt2[j]));
+        ssp = __dadd_rn(ssp, d);
+    }
+    #pragma unroll 4
+    for (int j = mp0; j <= mp1; ++j) {
+        const double d = value(j);
+        dmp = __dadd_rn(dmp, __dmul_rn(d, logt2[j]));
+        smp = __dadd_rn(smp, d);
+    }
+    if (pos_bits(sd)) {
+        double num = ssp;
+        if (weights) {
+            num = 0;
+            for (int j = 0; j < n; ++j) num = __dadd_rn(num, __dmul_rn(value(j), weights[j]));
+        }
+        o[0] = num / sd;
+        o[2] = smp / sd;
+    }
+    if (pos_bits(ssp)) o[1] = pm_exp(dsp / ssp);
+    if (pos_bits(smp)) o[3] = pm_exp(dmp / smp);
+}
+
+// Standalone T2partSEcorr (src/T2partSEcorr.jl:95-138): one thread per voxel, the
+// maps written in the call's type with NaN where the reference leaves them.
+// Bound by the FP64 pipe (64 cycles per instruction and 32 voxels), not by the
+// bytes it reads: so float values are widened on the integer pipes, unless the
+// voxel holds one that is not zero or normal, and 40 T2 times take ~190 instead
+// of 260 FP64 instructions: 240x240x16 voxels 488 us in 6 launches -> 345 us in one
+// (the call from host arrays 1.92 -> 1.75 ms, of 40x30x3 voxels 140 -> 109 us).
 template <class T>
 __global__ void k_t2part(const T *dist, long V, int n, int sp0, int sp1, int mp0, int mp1, const double *logt2,
-                         const double *weights, double *sfr, double *sgm, double *mfr, double *mgm) {
+                         const double *weights, T *sfr, T *sgm, T *mfr, T *mgm) {
     for (long v = blockIdx.x * (long)blockDim.x + threadIdx.x; v < V; v += (long)gridDim.x * blockDim.x) {
-        bool anynan = false;
-        for (int j = 0; j < n; ++j) anynan |= isnan((double)dist[v + V * j]);
-        if (anynan) continue;
-        double sd = 0, ssp = 0, smp = 0, dsp = 0, dmp = 0;
-        for (int j = 0; j < n; ++j) sd = __dadd_rn(sd, (double)dist[v + V * j]);
-        for (int j = sp0; j <= sp1; ++j) {
-            double d = dist[v + V * j];
-            dsp = __dadd_rn(dsp, __dmul_rn(d, logt2[j]));
-            ssp = __dadd_rn(ssp, d);
-        }
-        for (int j = mp0; j <= mp1; ++j) {
-            double d = dist[v + V * j];
-            dmp = __dadd_rn(dmp, __dmul_rn(d, logt2[j]));
-            smp = __dadd_rn(smp, d);
-        }
-        if (sd > 0) {
-            if (weights) {
-                double dw = 0;
-                for (int j = 0; j < n; ++j) dw = __dadd_rn(dw, __dmul_rn((double)dist[v + V * j], weights[j]));
-                sfr[v] = dw / sd;
+        double o[4] = {CUDART_NAN, CUDART_NAN, CUDART_NAN, CUDART_NAN};
+        bool anynan = false, odd = false;
+        #pragma unroll 4
+        for (int j = 0; j < n; ++j) {
+            if constexpr (sizeof(T) == 4) {
+                const unsigned u = __float_as_uint(dist[v + V * j]) & 0x7fffffffu;
+                anynan |= u > 0x7f800000u;
+                odd |= u - 1u < 0x7fffffu || u == 0x7f800000u;  // subnormal or infinite
             } else {
-                sfr[v] = ssp / sd;
+                anynan |= isnan_bits(dist[v + V * j]);
             }
-            mfr[v] = smp / sd;
         }
-        if (ssp > 0) sgm[v] = pm_exp(dsp / ssp);
-        if (smp > 0) mgm[v] = pm_exp(dmp / smp);
+        if (!anynan) {
+            auto plain = [&](int j) { return (double)dist[v + V * j]; };
+            if constexpr (sizeof(T) == 4) {
+                auto wide = [&](int j) { return widen(dist[v + V * j]); };
+                if (odd) t2part_voxel(plain, n, sp0, sp1, mp0, mp1, logt2, weights, o);
+                else t2part_voxel(wide, n, sp0, sp1, mp0, mp1, logt2, weights, o);
+            } else {
+                t2part_voxel(plain, n, sp0, sp1, mp0, mp1, logt2, weights, o);
+            }
+        }
+        sfr[v] = (T)o[0];
+        sgm[v] = (T)o[1];
+        mfr[v] = (T)o[2];
+        mgm[v] = (T)o[3];
     }
 }
 
-__global__ void k_narrow(const double *src, float *dst, long len) {
-    for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < len; i += (long)gridDim.x * blockDim.x)
-        dst[i] = (float)src[i];
+// FP64 buffers narrowed to float ones, all outputs of a call in one launch (a
+// block per kNarrowBlock values) instead of a launch each.
+constexpr int kNarrowMax = 17;
+constexpr long kNarrowBlock = 2048;
+struct NarrowJob {
+    const double *src[kNarrowMax];
+    float *dst[kNarrowMax];
+    long len[kNarrowMax];
+    long first[kNarrowMax + 1];  // first block of each
+    int n;
+};
+__global__ void __launch_bounds__(256) k_narrow(const __grid_constant__ NarrowJob J) {
+    int q = 0;
+    while (q + 1 < J.n && (long)blockIdx.x >= J.first[q + 1]) ++q;
+    const long i0 = ((long)blockIdx.x - J.first[q]) * kNarrowBlock, i1 = min(i0 + kNarrowBlock, J.len[q]);
+    const double *src = J.src[q];
+    float *dst = J.dst[q];
+    for (long i = i0 + threadIdx.x; i < i1; i += 256) dst[i] = (float)src[i];
 }
 
 }  // namespace dk
@@ -701,6 +754,22 @@ int out_layout(decaes_ctx *ctx, const decaes_t2map_opts &o, bool want_t2part, Ou
     return DECAES_OK;
 }
 
+// Collects FP64 outputs to be narrowed and launches them together.
+struct Narrow {
+    dk::NarrowJob J{};
+    void add(const double *src, float *dst, size_t len) {
+        if (!len) return;
+        J.src[J.n] = src; J.dst[J.n] = dst; J.len[J.n] = (long)len;
+        J.first[J.n + 1] = J.first[J.n] + ((long)len + dk::kNarrowBlock - 1) / dk::kNarrowBlock;
+        J.n++;
+    }
+    void launch(cudaStream_t st, int *launches) {
+        if (!J.n) return;
+        dk::k_narrow<<<(unsigned)J.first[J.n], 256, 0, st>>>(J);
+        ++*launches;
+    }
+};
+
 // Copy one device double output to a caller host buffer of the call dtype.
 int copy_out(decaes_ctx *ctx, const double *src, void *dst, size_t len, int dtype, cudaStream_t st, int *launches) {
     if (!dst || !src || !len) return DECAES_OK;
@@ -709,9 +778,9 @@ int copy_out(decaes_ctx *ctx, const double *src, void *dst, size_t len, int dtyp
     } else {
         void *tmp;
         if (int rc = buf(ctx, "narrow", sizeof(float) * len, &tmp)) return rc;
-        int g = (int)std::min<long>(8L * ctx->sms, ((long)len + 255) / 256);
-        dk::k_narrow<<<std::max(g, 1), 256, 0, st>>>(src, (float *)tmp, (long)len);
-        ++*launches;
+        Narrow nw;
+        nw.add(src, (float *)tmp, len);
+        nw.launch(st, launches);
         CK(cudaMemcpyAsync(dst, tmp, sizeof(float) * len, cudaMemcpyDeviceToHost, st));
         CK(cudaStreamSynchronize(st));  // `narrow` is reused by the next output
     }
@@ -840,10 +909,24 @@ static int t2map_host(decaes_ctx *ctx, const decaes_t2map_opts *mo, const decaes
         {om.alpha, mout->alpha, (size_t)V}, {om.resnorm, mout->resnorm, (size_t)V}, {om.decaycurve, mout->decaycurve, V * m},
         {om.mu, mout->mu, (size_t)V}, {om.chi2f, mout->chi2factor, (size_t)V}, {om.basis, mout->decaybasis, V * m * n},
     };
-    for (auto &c : cp)
-        if (int rc = copy_out(ctx, c.s, c.d, c.len, dtype, st, &launches)) return rc;
-    if (pout) {
-        struct { const double *s; void *d; } pc[] = {{om.sfr, pout->sfr}, {om.sgm, pout->sgm}, {om.mfr, pout->mfr}, {om.mgm, pout->mgm}};
+    struct { const double *s; void *d; } pc[] = {{om.sfr, pout ? pout->sfr : nullptr}, {om.sgm, pout ? pout->sgm : nullptr},
+                                                 {om.mfr, pout ? pout->mfr : nullptr}, {om.mgm, pout ? pout->mgm : nullptr}};
+    const DevBuf &nb = ctx->bufs["narrow"];
+    if (dtype == DECAES_F32 && (nb.bytes >= sizeof(float) * om.total || ctx->used - nb.bytes + sizeof(float) * om.total <= ctx->budget)) {
+        // all outputs narrowed in one launch, at their offsets, and copied without a wait between them
+        void *nf;
+        if (int rc = buf(ctx, "narrow", sizeof(float) * om.total, &nf)) return rc;
+        auto at = [&](const double *q) { return (float *)nf + (q - om.dist); };
+        Narrow nw;
+        for (auto &c : cp) if (c.s && c.d) nw.add(c.s, at(c.s), c.len);
+        for (auto &c : pc) if (c.s && c.d) nw.add(c.s, at(c.s), (size_t)V);
+        nw.launch(st, &launches);
+        CK(cudaGetLastError());
+        for (auto &c : cp) if (c.s && c.d && c.len) CK(cudaMemcpyAsync(c.d, at(c.s), sizeof(float) * c.len, cudaMemcpyDeviceToHost, st));
+        for (auto &c : pc) if (c.s && c.d) CK(cudaMemcpyAsync(c.d, at(c.s), sizeof(float) * (size_t)V, cudaMemcpyDeviceToHost, st));
+    } else {
+        for (auto &c : cp)
+            if (int rc = copy_out(ctx, c.s, c.d, c.len, dtype, st, &launches)) return rc;
         for (auto &c : pc)
             if (int rc = copy_out(ctx, c.s, c.d, (size_t)V, dtype, st, &launches)) return rc;
     }
@@ -921,24 +1004,19 @@ extern "C" int decaes_t2map_t2part_device(decaes_ctx *ctx, const decaes_t2map_op
         if (int rc = get_basis(ctx, o, &B)) return rc;
         fixed_basis = B->fixed;
     }
+    Narrow nw;
     for (auto &c : cp) {
         if (!c.s || !c.d) continue;
-        if (dtype == DECAES_F64) {
-            CK(cudaMemcpyAsync(c.d, c.s, sizeof(double) * c.len, cudaMemcpyDeviceToDevice, st));
-        } else {
-            int g = (int)std::min<long>(8L * ctx->sms, ((long)c.len + 255) / 256);
-            dk::k_narrow<<<std::max(g, 1), 256, 0, st>>>(c.s, (float *)c.d, (long)c.len);
-            ++launches;
-        }
+        if (dtype == DECAES_F64) CK(cudaMemcpyAsync(c.d, c.s, sizeof(double) * c.len, cudaMemcpyDeviceToDevice, st));
+        else nw.add(c.s, (float *)c.d, c.len);
     }
     if (fixed_basis) {
-        if (dtype == DECAES_F64) {
+        if (dtype == DECAES_F64)
             CK(cudaMemcpyAsync(d_mout->decaybasis, fixed_basis, sizeof(double) * m * n, cudaMemcpyDeviceToDevice, st));
-        } else {
-            dk::k_narrow<<<(int)((m * n + 255) / 256), 256, 0, st>>>(fixed_basis, (float *)d_mout->decaybasis, (long)(m * n));
-            ++launches;
-        }
+        else
+            nw.add(fixed_basis, (float *)d_mout->decaybasis, m * n);
     }
+    nw.launch(st, &launches);
     CK(cudaEventRecord(ctx->ev[5], st));
     CK(cudaGetLastError());
     ctx->stats.voxels = V;
@@ -985,7 +1063,7 @@ extern "C" int decaes_t2part(decaes_ctx *ctx, const decaes_t2part_opts *opts, co
     ctx->stats = decaes_stats{};
     void *d_dist, *d_out, *d_lt, *d_w = nullptr;
     if (int rc = buf(ctx, "t2p_dist", esize(dtype) * (size_t)V * n, &d_dist)) return rc;
-    if (int rc = buf(ctx, "t2p_out", sizeof(double) * 4 * (size_t)V, &d_out)) return rc;
+    if (int rc = buf(ctx, "t2p_out", esize(dtype) * 4 * (size_t)V, &d_out)) return rc;
     if (int rc = buf(ctx, "t2p_logt2", sizeof(double) * n, &d_lt)) return rc;
     if (!pp.weights.empty())
         if (int rc = buf(ctx, "t2p_w", sizeof(double) * n, &d_w)) return rc;
@@ -993,24 +1071,19 @@ extern "C" int decaes_t2part(decaes_ctx *ctx, const decaes_t2part_opts *opts, co
     CK(cudaMemcpyAsync(d_dist, dist, esize(dtype) * (size_t)V * n, cudaMemcpyHostToDevice, st));
     CK(cudaMemcpyAsync(d_lt, pp.logt2.data(), sizeof(double) * n, cudaMemcpyHostToDevice, st));
     if (d_w) CK(cudaMemcpyAsync(d_w, pp.weights.data(), sizeof(double) * n, cudaMemcpyHostToDevice, st));
-    double *po = (double *)d_out;
-    {
-        int g = (int)std::min<long>(8L * ctx->sms, (4 * V + 255) / 256);
-        dk::k_fill<<<std::max(g, 1), 256, 0, st>>>(po, 4 * V, NAN);
-        ++launches;
-    }
-    int g = (int)std::min<long>(8L * ctx->sms, (V + 127) / 128);
-    if (dtype == DECAES_F32)
-        dk::k_t2part<float><<<std::max(g, 1), 128, 0, st>>>((const float *)d_dist, V, n, pp.sp0, pp.sp1, pp.mp0, pp.mp1,
-                                                             (const double *)d_lt, (const double *)d_w, po, po + V, po + 2 * V, po + 3 * V);
-    else
-        dk::k_t2part<double><<<std::max(g, 1), 128, 0, st>>>((const double *)d_dist, V, n, pp.sp0, pp.sp1, pp.mp0, pp.mp1,
-                                                              (const double *)d_lt, (const double *)d_w, po, po + V, po + 2 * V, po + 3 * V);
+    int g = (int)std::min<long>(16L * ctx->sms, (V + 127) / 128);  // 64 warps per SM
+    auto run = [&](auto *src, auto *po) {
+        dk::k_t2part<<<std::max(g, 1), 128, 0, st>>>(src, V, n, pp.sp0, pp.sp1, pp.mp0, pp.mp1, (const double *)d_lt,
+                                                     (const double *)d_w, po, po + V, po + 2 * V, po + 3 * V);
+    };
+    if (dtype == DECAES_F32) run((const float *)d_dist, (float *)d_out);
+    else run((const double *)d_dist, (double *)d_out);
     ++launches;
     CK(cudaGetLastError());
     void *dsts[4] = {out->sfr, out->sgm, out->mfr, out->mgm};
+    const size_t ob = esize(dtype) * (size_t)V;
     for (int k = 0; k < 4; ++k)
-        if (int rc = copy_out(ctx, po + k * V, dsts[k], (size_t)V, dtype, st, &launches)) return rc;
+        if (dsts[k] && V) CK(cudaMemcpyAsync(dsts[k], (char *)d_out + k * ob, ob, cudaMemcpyDeviceToHost, st));
     CK(cudaEventRecord(ctx->ev[5], st));
     CK(cudaStreamSynchronize(st));
     float t;
@@ -1251,16 +1324,13 @@ int batch_enqueue(decaes_ctx *ctx, const BatchPrep &bp, cudaStream_t st, int *la
             {om.sfr, bv.t2part ? bv.v.d_pout.sfr : nullptr, V}, {om.sgm, bv.t2part ? bv.v.d_pout.sgm : nullptr, V},
             {om.mfr, bv.t2part ? bv.v.d_pout.mfr : nullptr, V}, {om.mgm, bv.t2part ? bv.v.d_pout.mgm : nullptr, V},
         };
+        Narrow nw;
         for (auto &c : cp) {
             if (!c.s || !c.d) continue;
-            if (bv.v.dtype == DECAES_F64) {
-                CK(cudaMemcpyAsync(c.d, c.s, sizeof(double) * c.len, cudaMemcpyDeviceToDevice, st));
-            } else {
-                int g = (int)std::min<long>(8L * ctx->sms, ((long)c.len + 255) / 256);
-                dk::k_narrow<<<std::max(g, 1), 256, 0, st>>>(c.s, (float *)c.d, (long)c.len);
-                ++*launches;
-            }
+            if (bv.v.dtype == DECAES_F64) CK(cudaMemcpyAsync(c.d, c.s, sizeof(double) * c.len, cudaMemcpyDeviceToDevice, st));
+            else nw.add(c.s, (float *)c.d, c.len);
         }
+        nw.launch(st, launches);
     }
     CK(cudaGetLastError());
     return DECAES_OK;
@@ -1652,16 +1722,17 @@ void srv_download(decaes_server *S, const ReqP &r) {
         {om.mfr, r->t2part ? r->pout.mfr : nullptr, V}, {om.mgm, r->t2part ? r->pout.mgm : nullptr, V},
     };
     bool ok = true;
+    auto narrowed = [&](const double *q) { return (float *)r->d_f32 + (q - r->d_out); };
+    if (r->dtype == DECAES_F32) {
+        Narrow nw;
+        int launches = 0;
+        for (auto &c : cp) if (c.s && c.d) nw.add(c.s, narrowed(c.s), c.len);
+        nw.launch(S->copy, &launches);
+    }
     for (auto &c : cp) {
         if (!c.s || !c.d || !ok) continue;
-        if (r->dtype == DECAES_F64) {
-            ok = cudaMemcpyAsync(c.d, c.s, sizeof(double) * c.len, cudaMemcpyDeviceToHost, S->copy) == cudaSuccess;
-        } else {
-            float *tmp = (float *)r->d_f32 + (c.s - r->d_out);
-            int g = (int)std::min<long>(8L * ctx->sms, ((long)c.len + 255) / 256);
-            dk::k_narrow<<<std::max(g, 1), 256, 0, S->copy>>>(c.s, tmp, (long)c.len);
-            ok = cudaMemcpyAsync(c.d, tmp, sizeof(float) * c.len, cudaMemcpyDeviceToHost, S->copy) == cudaSuccess;
-        }
+        ok = (r->dtype == DECAES_F64 ? cudaMemcpyAsync(c.d, c.s, sizeof(double) * c.len, cudaMemcpyDeviceToHost, S->copy)
+                                     : cudaMemcpyAsync(c.d, narrowed(c.s), sizeof(float) * c.len, cudaMemcpyDeviceToHost, S->copy)) == cudaSuccess;
     }
     if (ok) ok = cudaEventCreateWithFlags(&r->d2h, cudaEventDisableTiming) == cudaSuccess &&
                  cudaEventRecord(r->d2h, S->copy) == cudaSuccess;
