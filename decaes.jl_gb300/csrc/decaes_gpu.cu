@@ -586,6 +586,29 @@ int launch_wpb(decaes_ctx *ctx, const decaes_t2map_opts &o, Kern kern, long stri
     return o.legacy ? 1 : most_warps_wpb(ctx, kern, stride);
 }
 
+// Plain method: the rows of the NNLS matrix kept in shared memory.  The m + n
+// rows are reached only by solves with nearly every column in set P (one of ~33
+// in an L-curve voxel), so the last padding rows go to global scratch where that
+// lets one more warp live on an SM and leaves at least 0.6 n padding rows (below
+// that half the solves would leave shared memory).  FP64 method, 64x64x1 voxels:
+// 56 echoes x 60 T2 times (3 -> 4 warps) chi2 43.3 -> 36.1 ms, GCV 94.4 -> 77.4;
+// 48 x 48 (5 -> 6) L-curve 57.8 -> 49.0; 48 x 40 (7 -> 8) L-curve, 120x120x1,
+// 115.0 -> 113.0 ms.
+void spill_rows(decaes_ctx *ctx, int m, int n, dk::Params &P, long *wsm) {
+    constexpr int kMaxWarps = 8;  // of the plain kernel's block
+    const long avail = (long)(ctx->smem_optin / sizeof(double));
+    const long w = avail / *wsm + 1;
+    if (w < 2 || w > kMaxWarps) return;
+    const long fixed = dk::warp_smem_doubles(m, n, 0), per_warp = (avail / w) & ~1L;
+    long lda = (per_warp - fixed) / n;
+    if (lda % 2 == 0) lda -= 1;  // odd: no bank conflicts down or across columns
+    if (lda < m + (3L * n + 4) / 5 || lda < (std::max(m, n) | 1)) return;
+    P.lda = (int)lda;
+    P.epg_lanes = dk::fp64_epg_lanes(m, n, P.lda);
+    P.scr_stride += dk::warp_spill_doubles(m, n, P.lda);
+    *wsm = (dk::warp_smem_doubles(m, n, P.lda) + 1) & ~1L;
+}
+
 // Persistent grid for a kernel whose warps each need `stride` doubles of
 // shared memory: blocks of wpb warps, as many as fit on every SM at once, or
 // at most bps of them per SM when bps > 0.
@@ -630,6 +653,7 @@ int run_t2map(decaes_ctx *ctx, const decaes_t2map_opts &o, const decaes_t2part_o
     dk::Params P;
     long wsm = 0;
     if (int rc = make_params(ctx, o, po ? &pp : nullptr, d_weights, B, d_image, dtype, d_b1, out, P, &wsm)) return rc;
+    if (!P.mixed && !o.legacy && tuned_wpb_or0(ctx, o) == 0) spill_rows(ctx, o.nTE, n, P, &wsm);
     // NaN-fill outputs
     {
         int g = std::min<long>(4L * ctx->sms * 8, (long)(out.total + 255) / 256);

@@ -240,7 +240,24 @@ struct NnlsWS {
     ShI posof;               // n, 1-based logical position of each physical column (inverse of idx)
     ShI zl;                  // n, scratch list of physical columns
     int lda;
+    // rows lim + 1 .. lim + lsp of the columns (the last padding rows, which only
+    // solves with nearly every column in set P reach) in global scratch
+    int lim, lsp;
+    double *sp;
 };
+// Row i (1-based) of physical column p, and the same past lim.  kSpill: the call
+// may reach such rows (out-of-line copies for those calls, so that the others
+// test nothing per row).
+__device__ __forceinline__ double *spilled(const NnlsWS &s, int p) { return s.sp + (long)p * s.lsp - s.lim - 1; }  // [i], i > lim
+template <bool kSpill>
+__device__ __forceinline__ double row_get(const NnlsWS &s, int p, int i) {
+    return !kSpill || i <= s.lim ? s.C[i - 1 + p * s.lda] : spilled(s, p)[i];
+}
+template <bool kSpill>
+__device__ __forceinline__ void row_set(const NnlsWS &s, int p, int i, double v) {
+    if (!kSpill || i <= s.lim) s.C[i - 1 + p * s.lda] = v;
+    else spilled(s, p)[i] = v;
+}
 
 // Physical columns whose logical position is >= jfirst, in increasing
 // physical order, written to s.zl; returns their count.  Column-parallel
@@ -273,11 +290,6 @@ __device__ __forceinline__ double mdiv(double a, double b, double r) {
     return fma(e, r, q);
 }
 
-__device__ __forceinline__ double &Aat(const NnlsWS &s, int i1, int j1) {
-    // 1-based row i1 of logical column j1
-    return s.C[(i1 - 1) + (s.idx[j1 - 1] - 1) * s.lda];
-}
-
 // Base.hypot for Float64 (C. F. Borges, "An Improved Algorithm for
 // hypot(a,b)", 2019, fma-corrected), used by NNLS.orthogonal_rotmat.
 static __device__ double jl_hypot(double x, double y) {
@@ -301,14 +313,16 @@ static __device__ double jl_hypot(double x, double y) {
 
 // construct_apply_householder!(A, b, ip, jp, m), src/NNLS.jl:259-336.
 // Writes only the pivot column's physical storage (see header note).
-static __device__ double warp_cah(const NnlsWS &s, int ip, int jp, int m) {
+template <bool kSpill>
+__device__ __forceinline__ double warp_cah_t(const NnlsWS &s, int ip, int jp, int m) {
     const int lane = threadIdx.x & 31;
     if (ip > m) return 0.0;
-    const ShD col = s.C + (s.idx[jp - 1] - 1) * s.lda;  // pivot column (0-based rows)
+    const int pc = s.idx[jp - 1] - 1;  // pivot column
+    const ShD col = s.C + pc * s.lda;
     double alpha = col[ip - 1];
     double part = 0.0;
     #pragma unroll 1
-    for (int i = ip + lane; i <= m; i += 32) part = fma(col[i - 1], col[i - 1], part);
+    for (int i = ip + lane; i <= m; i += 32) { const double v = row_get<kSpill>(s, pc, i); part = fma(v, v, part); }
     double xnorm = sqrt(wsum(part));
     if ((__double_as_longlong(xnorm) << 1) == 0) return -1.0;  // xnorm == 0
     double beta = copysign(xnorm, alpha);
@@ -322,7 +336,7 @@ static __device__ double warp_cah(const NnlsWS &s, int ip, int jp, int m) {
     part = 0.0;
     #pragma unroll 1
     for (int i = ip + 1 + lane; i <= m; i += 32) {
-        double qi = mdiv(col[i - 1], alpha, ralpha);
+        double qi = mdiv(row_get<kSpill>(s, pc, i), alpha, ralpha);
         s.zz[i - 1] = qi;
         part = fma(s.b[i - 1], qi, part);
     }
@@ -343,7 +357,7 @@ static __device__ double warp_cah(const NnlsWS &s, int ip, int jp, int m) {
             #pragma unroll 1
             for (int i = ip + 1 + lane; i <= m; i += 32) {
                 double qi = s.zz[i - 1];
-                col[i - 1] = qi;
+                row_set<kSpill>(s, pc, i, qi);
                 s.b[i - 1] = fma(sm, qi, s.b[i - 1]);
             }
             const double rA1 = -rbeta;  // 1 / (-beta), exact negation
@@ -364,16 +378,24 @@ static __device__ double warp_cah(const NnlsWS &s, int ip, int jp, int m) {
     return -1.0;
 }
 
+static __device__ __noinline__ double warp_cah_spill(const NnlsWS s, int ip, int jp, int m) { return warp_cah_t<true>(s, ip, jp, m); }
+__device__ __forceinline__ double warp_cah(const NnlsWS &s, int ip, int jp, int m) {
+    return m > s.lim ? warp_cah_spill(s, ip, jp, m) : warp_cah_t<false>(s, ip, jp, m);
+}
+
 // apply_householder_dual!(A, w, b, tau, j1, m1), src/NNLS.jl:379-436.
 // Lanes over logical columns j1+1..n; a column's two sums run down its rows in
 // one lane.  A round of at most 16 columns spreads the update between them over
 // all lanes, (column, row) pairs at a time: with 8 columns 2.25 instead of 3
 // FP64 warp instructions per row: 120x120x1 x 48 echoes, L-curve, 125.5 -> 120.1
 // ms; 32x32x4 x 32 echoes, chi2, 17.3 -> 16.75 ms.
-static __device__ void warp_ahd(const NnlsWS &s, int n, double tau, int j1, int m1) {
+template <bool kSpill>
+__device__ __forceinline__ void warp_ahd_t(const NnlsWS &s, int n, double tau, int j1, int m1) {
     const int lane = threadIdx.x & 31;
     if (j1 >= m1) return;
-    const ShD u = s.C + (s.idx[j1 - 1] - 1) * s.lda;  // u[j1-1] is the diagonal; treated as 1
+    const int pu = s.idx[j1 - 1] - 1, mi = kSpill ? min(m1, s.lim) : m1;  // rows up to mi in shared memory
+    const ShD u = s.C + pu * s.lda;                          // u[j1-1] is the diagonal; treated as 1
+    const double *us = spilled(s, pu);
     const int nz = warp_active_cols(s, n, j1 + 1);
     #pragma unroll 1
     for (int r0 = 0; r0 < nz; r0 += 32) {
@@ -381,11 +403,14 @@ static __device__ void warp_ahd(const NnlsWS &s, int n, double tau, int j1, int 
         const bool mine = r < nz;
         const int p = mine ? s.zl[r] : 0;
         const ShD a = s.C + p * s.lda;
+        double *as = spilled(s, p);
         double sm = 0.0;
         if (mine) {
             sm = fma(a[j1 - 1], 1.0, 0.0);
             #pragma unroll 8
-            for (int i = j1 + 1; i <= m1; ++i) sm = fma(a[i - 1], u[i - 1], sm);
+            for (int i = j1 + 1; i <= mi; ++i) sm = fma(a[i - 1], u[i - 1], sm);
+            #pragma unroll 1
+            for (int i = mi + 1; kSpill && i <= m1; ++i) sm = fma(as[i], us[i], sm);
             sm *= -tau;
             a[j1 - 1] = a[j1 - 1] + sm;
         }
@@ -393,10 +418,16 @@ static __device__ void warp_ahd(const NnlsWS &s, int n, double tau, int j1, int 
             if (mine) {
                 double wj = 0.0;
                 #pragma unroll 8
-                for (int i = j1 + 1; i <= m1; ++i) {
+                for (int i = j1 + 1; i <= mi; ++i) {
                     double v = fma(sm, u[i - 1], a[i - 1]);
                     wj = fma(v, s.b[i - 1], wj);
                     a[i - 1] = v;
+                }
+                #pragma unroll 1
+                for (int i = mi + 1; kSpill && i <= m1; ++i) {
+                    double v = fma(sm, us[i], as[i]);
+                    wj = fma(v, s.b[i - 1], wj);
+                    as[i] = v;
                 }
                 s.w[s.posof[p] - 1] = wj;
             }
@@ -406,15 +437,22 @@ static __device__ void warp_ahd(const NnlsWS &s, int n, double tau, int j1, int 
             __syncwarp();
             const double smc = __shfl_sync(FULL, sm, c);
             if (c < cnt) {
-                const ShD ac = s.C + s.zl[r0 + c] * s.lda;
+                const int q = s.zl[r0 + c];
+                const ShD ac = s.C + q * s.lda;
+                double *acs = spilled(s, q);
+                int i = j1 + 1 + (lane >> lg);
                 #pragma unroll 4
-                for (int i = j1 + 1 + (lane >> lg); i <= m1; i += 32 >> lg) ac[i - 1] = fma(smc, u[i - 1], ac[i - 1]);
+                for (; i <= mi; i += 32 >> lg) ac[i - 1] = fma(smc, u[i - 1], ac[i - 1]);
+                #pragma unroll 1
+                for (; kSpill && i <= m1; i += 32 >> lg) acs[i] = fma(smc, us[i], acs[i]);
             }
             __syncwarp();
             if (mine) {
                 double wj = 0.0;
                 #pragma unroll 8
-                for (int i = j1 + 1; i <= m1; ++i) wj = fma(a[i - 1], s.b[i - 1], wj);
+                for (int i = j1 + 1; i <= mi; ++i) wj = fma(a[i - 1], s.b[i - 1], wj);
+                #pragma unroll 1
+                for (int i = mi + 1; kSpill && i <= m1; ++i) wj = fma(as[i], s.b[i - 1], wj);
                 s.w[s.posof[p] - 1] = wj;
             }
         }
@@ -422,23 +460,39 @@ static __device__ void warp_ahd(const NnlsWS &s, int n, double tau, int j1, int 
     __syncwarp();
 }
 
+static __device__ __noinline__ void warp_ahd_spill(const NnlsWS s, int n, double tau, int j1, int m1) { warp_ahd_t<true>(s, n, tau, j1, m1); }
+__device__ __forceinline__ void warp_ahd(const NnlsWS &s, int n, double tau, int j1, int m1) {
+    if (m1 > s.lim) warp_ahd_spill(s, n, tau, j1, m1);
+    else warp_ahd_t<false>(s, n, tau, j1, m1);
+}
+
 // compute_dual!(w, A, b, j1, m1), src/NNLS.jl:441-470.  Lanes over columns.
-static __device__ void warp_compute_dual(const NnlsWS &s, int n, int j1, int m1) {
+template <bool kSpill>
+__device__ __forceinline__ void warp_compute_dual_t(const NnlsWS &s, int n, int j1, int m1) {
     const int lane = threadIdx.x & 31;
-    const int nz = warp_active_cols(s, n, j1);
+    const int nz = warp_active_cols(s, n, j1), mi = kSpill ? min(m1, s.lim) : m1;
     #pragma unroll 1
     for (int r0 = 0; r0 < nz; r0 += 32) {
         int r = r0 + lane;
         if (r < nz) {
             const int p = s.zl[r];
             const ShD a = s.C + p * s.lda;
+            const double *as = spilled(s, p);
             double sm = 0.0;
             #pragma unroll 8
-            for (int i = j1; i <= m1; ++i) sm = fma(a[i - 1], s.b[i - 1], sm);
+            for (int i = j1; i <= mi; ++i) sm = fma(a[i - 1], s.b[i - 1], sm);
+            #pragma unroll 1
+            for (int i = mi + 1; kSpill && i <= m1; ++i) sm = fma(as[i], s.b[i - 1], sm);
             s.w[s.posof[p] - 1] = sm;
         }
     }
     __syncwarp();
+}
+
+static __device__ __noinline__ void warp_compute_dual_spill(const NnlsWS s, int n, int j1, int m1) { warp_compute_dual_t<true>(s, n, j1, m1); }
+__device__ __forceinline__ void warp_compute_dual(const NnlsWS &s, int n, int j1, int m1) {
+    if (m1 > s.lim) warp_compute_dual_spill(s, n, j1, m1);
+    else warp_compute_dual_t<false>(s, n, j1, m1);
 }
 
 // zz[1:n] = b[1:n]; solve_triangular_system!(zz, A, n), src/NNLS.jl:506-523.
@@ -487,23 +541,6 @@ static __device__ void warp_solve_tri(const NnlsWS &s, int n) {
     }
 }
 
-// Transposed solve (U' z = x) on the first n logical columns, src/NNLS.jl:524-537.
-static __device__ void warp_solve_tri_t(const NnlsWS &s, ShD z, int n) {
-    const int lane = threadIdx.x & 31;
-    #pragma unroll 1
-    for (int j = 1; j <= n; ++j) {
-        const ShD a = s.C + (s.idx[j - 1] - 1) * s.lda;
-        double part = 0.0;
-        #pragma unroll 1
-        for (int l = 1 + lane; l <= j - 1; l += 32) part = fma(-a[l - 1], z[l - 1], part);
-        double z1 = z[j - 1] + wsum(part);
-        z1 /= a[j - 1];
-        __syncwarp();
-        if (lane == 0) z[j - 1] = z1;
-        __syncwarp();
-    }
-}
-
 // Logical position j1..n of the largest positive dual (the first one, as the
 // reference's `w[j] > wmax` scan from wmax = 0), 0 when there is none.  Positive
 // doubles order like their bit patterns, so the search runs on the integer pipes.
@@ -545,7 +582,7 @@ static __device__ NnlsResult warp_nnls(const NnlsWS &s, int M, int n, int m0, bo
             jmax = warp_largest_dual(s, n, nsetp + 1);
             if (jmax == 0) { terminated = true; break; }  // no positive dual
             if (tikh && !s.diag[s.idx[jmax - 1] - 1]) {
-                if (lane == 0) Aat(s, m + 1, jmax) = lam;
+                if (lane == 0) row_set<true>(s, s.idx[jmax - 1] - 1, m + 1, lam);
                 __syncwarp();
             }
             tau = warp_cah(s, nsetp + 1, jmax, tikh ? min(m + 1, M) : m);
@@ -553,7 +590,7 @@ static __device__ NnlsResult warp_nnls(const NnlsWS &s, int M, int n, int m0, bo
             __syncwarp();
             if (lane == 0) {
                 s.w[jmax - 1] = 0.0;
-                if (tikh && m < M) Aat(s, m + 1, jmax) = 0.0;
+                if (tikh && m < M) row_set<true>(s, s.idx[jmax - 1] - 1, m + 1, 0.0);
             }
             __syncwarp();
         }
@@ -575,9 +612,9 @@ static __device__ NnlsResult warp_nnls(const NnlsWS &s, int M, int n, int m0, bo
         __syncwarp();
         if (nsetp < n) warp_ahd(s, n, tau, nsetp, m);
         {
-            const ShD pc = s.C + (s.idx[nsetp - 1] - 1) * s.lda;
+            const int pc = s.idx[nsetp - 1] - 1;
             #pragma unroll 1
-            for (int i = nsetp + 1 + lane; i <= m; i += 32) pc[i - 1] = 0.0;
+            for (int i = nsetp + 1 + lane; i <= m; i += 32) row_set<true>(s, pc, i, 0.0);
         }
         __syncwarp();
         if (lane == 0) s.w[nsetp - 1] = 0.0;
@@ -727,7 +764,7 @@ static __device__ __noinline__ NnlsResult warp_lsq(const NnlsWS s, const double 
         #pragma unroll 1
         for (int i = lane; i < m; i += 32) copy_async(cj + i, aj + i);
         #pragma unroll 1
-        for (int i = m + lane; i < M; i += 32) cj[i] = 0.0;
+        for (int i = m + lane; i < M; i += 32) row_set<true>(s, j, i + 1, 0.0);
     }
     #pragma unroll 1
     for (int i = lane; i < M; i += 32) s.b[i] = (i < m) ? data[i] : 0.0;

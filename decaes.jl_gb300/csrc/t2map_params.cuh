@@ -9,7 +9,8 @@ constexpr int kLoopCap = 512;    // hard cap of every data-dependent outer loop
 constexpr int kSolCap = 64;      // stored Tikhonov solutions per voxel (keyed by log mu)
 
 struct Params {
-    int m, n, K, M, lda;
+    int m, n, K, M;
+    int lda;  // plain method: matrix rows in shared memory, the leading dimension
     int reg;
     double chi2factor, noiselevel;
     int mineval, maxeval;
@@ -65,8 +66,10 @@ struct BatchParams {
 };
 
 // Shared-memory footprint of one warp worker (doubles), mirrored on the host.
+// lda: the matrix's rows in shared memory, at least max(m, n) | 1 (the rest of
+// the m + n rows, the last padding rows, in the warp's global scratch).
 __host__ __device__ inline long warp_smem_doubles(int m, int n, int lda) {
-    long d = (long)lda * n + 3L * lda + 4L * n + 8;
+    long d = (long)lda * n + 2L * ((m + n) | 1) + m + 4L * n + 8;
     long ints = 4L * n;            // idx, posof, zl
     long bytes = (long)n;          // diag
     return d + (ints * 4 + bytes + 7) / 8;
@@ -114,5 +117,7 @@ __host__ __device__ inline long warp_scratch_f32_offset(int m, int n, int K) {
 __host__ __device__ inline long warp_scratch_doubles(int m, int n, int K) {
     return warp_scratch_f32_offset(m, n, K) + ((long)m * n + 1) / 2;
 }
+// The plain method's matrix rows past lda follow it.
+__host__ __device__ inline long warp_spill_doubles(int m, int n, int lda) { return m + n > lda ? (long)(m + n - lda) * n : 0; }
 
 }  // namespace dk

@@ -44,9 +44,10 @@ static __device__ void warp_setup(Warp &w, const Params &P, ShD p, double *scr) 
         w.s.lda = lda;
     } else {
         w.s.C = p; p += lda * n;
-        w.s.b = p; p += lda;
-        w.s.zz = p; p += lda;
-        w.data = p; p += lda;
+        const int M = P.m + n;
+        w.s.b = p; p += M | 1;
+        w.s.zz = p; p += M | 1;
+        w.data = p; p += P.m;
         w.s.x = p; p += n;
         w.s.w = p; p += n;
         w.xout = p; p += n;
@@ -57,6 +58,9 @@ static __device__ void warp_setup(Warp &w, const Params &P, ShD p, double *scr) 
         w.s.zl = w.s.posof + n;
         w.s.diag = (w.s.zl + 2 * n).as<unsigned char>();
         w.s.lda = lda;
+        w.s.lim = M < lda ? M : lda;
+        w.s.lsp = M - w.s.lim;
+        w.s.sp = scr + warp_scratch_doubles(P.m, n, P.K);
     }
     w.scr = scr;
     const int mn = P.m < P.n ? P.m : P.n;
