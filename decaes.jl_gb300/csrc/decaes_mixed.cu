@@ -1,7 +1,8 @@
 // decaes_mixed.cu -- the voxel-solve kernel with the mixed-precision method only: single-volume launches
 // and batched / served launches whose volumes all use that method run these
 // kernels (half the code of the kernels that carry both methods).  A separate
-// translation unit, compiled in parallel with the others.
+// translation unit, compiled in parallel with the others.  512 threads: one block
+// holds up to 16 warps, as many as an SM's registers and shared memory take.
 #define DECAES_METHODS 2
 #include "voxel_kernels.cuh"
 

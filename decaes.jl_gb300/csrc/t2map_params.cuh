@@ -108,7 +108,8 @@ __host__ __device__ inline int fp64_epg_lanes(int m, int n, int lda) {
 }
 // Global scratch of one warp worker (doubles).
 // Offset of the mixed method's FP32 basis (m x n floats) in it, after the
-// per-voxel basis, surrogate samples, L-curve caches, singular values and the
+// per-voxel basis, surrogate samples, L-curve caches (kCacheCap * 19 doubles: the
+// legacy algorithms' workspace lies there too and sets the size), singular values and the
 // stored solutions.
 __host__ __device__ inline long warp_scratch_f32_offset(int m, int n, int K) {
     int mn = m < n ? m : n;
