@@ -24,6 +24,7 @@
 
 #include "decaes_gpu.h"
 #include "decaes_tc.h"
+#include "devpool.h"
 #include "epg.cuh"
 #include "host.h"
 #include "voxel_kernels.cuh"
@@ -278,11 +279,6 @@ int raise_smem_limit(const void *kern, size_t bytes) {
 
 namespace {
 
-struct DevBuf {
-    void *p = nullptr;
-    size_t bytes = 0;
-};
-
 struct BasisKey {
     int m, n, K, beta180;
     double TE, T1, t2lo, t2hi, minang, beta, fixed;
@@ -330,7 +326,7 @@ struct decaes_ctx {
     cudaEvent_t ev[8];
     std::string err;
     decaes_stats stats{};
-    std::map<std::string, DevBuf> bufs;
+    std::map<std::string, dh::DevBuf> bufs;
     std::map<BasisKey, Basis> bases;
     long tick = 0;
     int sms = 0;
@@ -356,21 +352,39 @@ int fail(decaes_ctx *c, int code, const std::string &msg) {
         if (e_ != cudaSuccess) return fail(ctx, DECAES_ECUDA, std::string(#call) + ": " + cudaGetErrorString(e_)); \
     } while (0)
 
+// The allocator of the context's buffers; `e` keeps the last refusal, which is
+// taken off the runtime's error state (callers may go on without the memory).
+struct DevAlloc {
+    cudaError_t *e;
+    bool operator()(void **p, size_t bytes) const {
+        *e = cudaMalloc(p, bytes);
+        if (*e == cudaSuccess) return true;
+        cudaGetLastError();
+        *p = nullptr;
+        return false;
+    }
+};
+void dev_free(void *p) { cudaFree(p); }
+bool fits(decaes_ctx *ctx, size_t bytes) { return dh::pool_fits(*ctx, bytes, dev_free); }
+cudaError_t dev_alloc(decaes_ctx *ctx, void **p, size_t bytes) {
+    cudaError_t e = cudaSuccess;
+    return dh::pool_alloc(*ctx, p, bytes, DevAlloc{&e}, dev_free) ? cudaSuccess : e;
+}
+template <class T>
+cudaError_t dev_alloc(decaes_ctx *ctx, T **p, size_t bytes) {
+    return dev_alloc(ctx, reinterpret_cast<void **>(p), bytes);
+}
+
 // Grow-only named device buffers, accounted against the HBM budget.
 int buf(decaes_ctx *ctx, const std::string &name, size_t bytes, void **out) {
-    DevBuf &b = ctx->bufs[name];
-    if (b.bytes < bytes) {
-        if (b.p) { cudaFree(b.p); ctx->used -= b.bytes; b.p = nullptr; b.bytes = 0; }
-        if (ctx->used + bytes > ctx->budget)
+    cudaError_t e = cudaSuccess;
+    switch (dh::pool_get(*ctx, name, bytes, DevAlloc{&e}, dev_free, out)) {
+        case dh::kPoolOk: return DECAES_OK;
+        case dh::kPoolOverBudget:
             return fail(ctx, DECAES_ENOMEM, "device allocation of " + std::to_string(bytes) + " bytes for '" + name +
                                                 "' exceeds the context's HBM budget");
-        cudaError_t e = cudaMalloc(&b.p, bytes);
-        if (e != cudaSuccess) return fail(ctx, DECAES_ECUDA, std::string("cudaMalloc: ") + cudaGetErrorString(e));
-        b.bytes = bytes;
-        ctx->used += bytes;
+        default: return fail(ctx, DECAES_ECUDA, std::string("cudaMalloc: ") + cudaGetErrorString(e));
     }
-    *out = b.p;
-    return DECAES_OK;
 }
 
 size_t esize(int dtype) { return dtype == DECAES_F32 ? 4 : 8; }
@@ -410,23 +424,23 @@ int get_basis(decaes_ctx *ctx, const decaes_t2map_opts &o, Basis **out) {
     b.h_angles = fixed ? std::vector<double>{o.SetFlipAngle} : dh::julia_range(o.MinRefAngle, 180.0, K);
     size_t mnk = (size_t)m * n * K;
     b.bytes = sizeof(double) * (2 * n + K + (fixed ? (size_t)m * n : 2 * mnk));
-    if (ctx->used + b.bytes > ctx->budget) return fail(ctx, DECAES_ENOMEM, "resident basis exceeds the HBM budget");
-    CK(cudaMalloc(&b.t2, sizeof(double) * n));
-    CK(cudaMalloc(&b.logt2, sizeof(double) * n));
-    CK(cudaMalloc(&b.angles, sizeof(double) * K));
+    if (!fits(ctx, b.bytes)) return fail(ctx, DECAES_ENOMEM, "resident basis exceeds the HBM budget");
+    CK(dev_alloc(ctx, &b.t2, sizeof(double) * n));
+    CK(dev_alloc(ctx, &b.logt2, sizeof(double) * n));
+    CK(dev_alloc(ctx, &b.angles, sizeof(double) * K));
     CK(cudaMemcpyAsync(b.t2, b.h_t2.data(), sizeof(double) * n, cudaMemcpyHostToDevice, ctx->stream));
     CK(cudaMemcpyAsync(b.logt2, logt2.data(), sizeof(double) * n, cudaMemcpyHostToDevice, ctx->stream));
     CK(cudaMemcpyAsync(b.angles, b.h_angles.data(), sizeof(double) * K, cudaMemcpyHostToDevice, ctx->stream));
     const int beta180 = o.RefConAngle == 180.0;
     if (fixed) {
-        CK(cudaMalloc(&b.fixed, sizeof(double) * m * n));
+        CK(dev_alloc(ctx, &b.fixed, sizeof(double) * m * n));
         void *work;
         if (int rc = buf(ctx, "epgwork", sizeof(double) * 3 * (size_t)m * n, &work)) return rc;
         dk::k_basis_fixed<<<(n + 63) / 64, 64, 0, ctx->stream>>>(m, n, o.SetFlipAngle, o.TE, o.T1, beta180, o.RefConAngle,
                                                                  b.t2, b.fixed, (double *)work);
     } else {
-        CK(cudaMalloc(&b.As, sizeof(double) * mnk));
-        CK(cudaMalloc(&b.dAs, sizeof(double) * mnk));
+        CK(dev_alloc(ctx, &b.As, sizeof(double) * mnk));
+        CK(dev_alloc(ctx, &b.dAs, sizeof(double) * mnk));
         void *work;
         if (int rc = buf(ctx, "epgwork", sizeof(dx::Dual) * 4 * (size_t)m * n * K, &work)) return rc;
         dk::k_ensemble<<<(n * K + 63) / 64, 64, 0, ctx->stream>>>(m, n, K, o.TE, o.T1, beta180, o.RefConAngle, b.t2,
@@ -466,9 +480,9 @@ int prepare_basis(decaes_ctx *ctx, const decaes_t2map_opts &o, cudaStream_t st, 
     if (mixed && !B->Gs) {
         const int K = fixed ? 1 : o.nRefAngles;
         const size_t gb = sizeof(double) * (size_t)K * (n * (n + 1) / 2), tb = sizeof(double) * (size_t)K * m * n;
-        if (ctx->used + gb + tb > ctx->budget) return fail(ctx, DECAES_ENOMEM, "Gram matrices exceed the HBM budget");
-        CK(cudaMalloc(&B->Gs, gb));
-        CK(cudaMalloc(&B->AsT, tb));
+        if (!fits(ctx, gb + tb)) return fail(ctx, DECAES_ENOMEM, "Gram matrices exceed the HBM budget");
+        CK(dev_alloc(ctx, &B->Gs, gb));
+        CK(dev_alloc(ctx, &B->AsT, tb));
         B->bytes += gb + tb;
         ctx->used += gb + tb;
         dk::k_gram_grid<<<K, 256, 0, ctx->stream>>>(m, n, fixed ? B->fixed : B->As, B->Gs, B->AsT);
@@ -479,8 +493,8 @@ int prepare_basis(decaes_ctx *ctx, const decaes_t2map_opts &o, cudaStream_t st, 
     if (o.precision == DECAES_PREC_MIXED_TC && !fixed && !B->Bsl) {
         const int K = o.nRefAngles;
         const size_t sb = (size_t)dk::tc_ntiles(K, n) * dk::kTcSlices * dk::tc_slice_bytes(dk::kTcTileN, dk::tc_mpad(m));
-        if (ctx->used + sb > ctx->budget) return fail(ctx, DECAES_ENOMEM, "grid-basis slices exceed the HBM budget");
-        CK(cudaMalloc(&B->Bsl, sb));
+        if (!fits(ctx, sb)) return fail(ctx, DECAES_ENOMEM, "grid-basis slices exceed the HBM budget");
+        CK(dev_alloc(ctx, &B->Bsl, sb));
         B->bytes += sb;
         ctx->used += sb;
         CK(dk::tc_make_basis_slices(B->As, m, n, K, B->Bsl, ctx->stream));
@@ -801,7 +815,7 @@ int copy_out(decaes_ctx *ctx, const double *src, void *dst, size_t len, int dtyp
         CK(cudaMemcpyAsync(dst, src, sizeof(double) * len, cudaMemcpyDeviceToHost, st));
     } else {
         void *tmp;
-        if (int rc = buf(ctx, "narrow", sizeof(float) * len, &tmp)) return rc;
+        if (int rc = buf(ctx, dh::kNarrowBuf, sizeof(float) * len, &tmp)) return rc;
         Narrow nw;
         nw.add(src, (float *)tmp, len);
         nw.launch(st, launches);
@@ -935,19 +949,27 @@ static int t2map_host(decaes_ctx *ctx, const decaes_t2map_opts *mo, const decaes
     };
     struct { const double *s; void *d; } pc[] = {{om.sfr, pout ? pout->sfr : nullptr}, {om.sgm, pout ? pout->sgm : nullptr},
                                                  {om.mfr, pout ? pout->mfr : nullptr}, {om.mgm, pout ? pout->mgm : nullptr}};
-    const DevBuf &nb = ctx->bufs["narrow"];
-    if (dtype == DECAES_F32 && (nb.bytes >= sizeof(float) * om.total || ctx->used - nb.bytes + sizeof(float) * om.total <= ctx->budget)) {
-        // all outputs narrowed in one launch, at their offsets, and copied without a wait between them
-        void *nf;
-        if (int rc = buf(ctx, "narrow", sizeof(float) * om.total, &nf)) return rc;
-        auto at = [&](const double *q) { return (float *)nf + (q - om.dist); };
+    // a float call's requested outputs narrowed in one launch, packed, and copied
+    // without a wait between them; one by one when there is no room for all
+    std::vector<std::tuple<const double *, void *, size_t>> want;
+    size_t joint = 0;
+    if (dtype == DECAES_F32) {
+        for (auto &c : cp) if (c.s && c.d && c.len) { want.emplace_back(c.s, c.d, c.len); joint += c.len; }
+        for (auto &c : pc) if (c.s && c.d && V) { want.emplace_back(c.s, c.d, (size_t)V); joint += (size_t)V; }
+    }
+    void *nf = nullptr;
+    cudaError_t ne = cudaSuccess;
+    if (joint && dh::pool_get(*ctx, dh::kNarrowBuf, sizeof(float) * joint, DevAlloc{&ne}, dev_free, &nf) == dh::kPoolOk) {
         Narrow nw;
-        for (auto &c : cp) if (c.s && c.d) nw.add(c.s, at(c.s), c.len);
-        for (auto &c : pc) if (c.s && c.d) nw.add(c.s, at(c.s), (size_t)V);
+        float *f = (float *)nf;
+        for (auto &[src, dst, len] : want) { nw.add(src, f, len); f += len; }
         nw.launch(st, &launches);
         CK(cudaGetLastError());
-        for (auto &c : cp) if (c.s && c.d && c.len) CK(cudaMemcpyAsync(c.d, at(c.s), sizeof(float) * c.len, cudaMemcpyDeviceToHost, st));
-        for (auto &c : pc) if (c.s && c.d) CK(cudaMemcpyAsync(c.d, at(c.s), sizeof(float) * (size_t)V, cudaMemcpyDeviceToHost, st));
+        f = (float *)nf;
+        for (auto &[src, dst, len] : want) {
+            CK(cudaMemcpyAsync(dst, f, sizeof(float) * len, cudaMemcpyDeviceToHost, st));
+            f += len;
+        }
     } else {
         for (auto &c : cp)
             if (int rc = copy_out(ctx, c.s, c.d, c.len, dtype, st, &launches)) return rc;
@@ -1422,13 +1444,13 @@ extern "C" decaes_batch *decaes_batch_create(decaes_ctx *ctx, const decaes_volum
     if (int rc = batch_plan(ctx, vols, nvol, ctx->stream, b->bp, &launches)) return bail(rc);
     size_t sz[5];
     const size_t total = batch_bytes(b->bp, &sz[0], &sz[1], &sz[2], &sz[3], &sz[4]);
-    if (ctx->used + total > ctx->budget) {
+    if (!fits(ctx, total)) {
         fail(ctx, DECAES_ENOMEM, "the batch's working buffers (" + std::to_string(total) + " bytes) exceed the HBM budget");
         return bail(DECAES_ENOMEM);
     }
     void *p[5];
     for (int i = 0; i < 5; ++i) {
-        cudaError_t e = cudaMalloc(&p[i], sz[i]);
+        cudaError_t e = dev_alloc(ctx, &p[i], sz[i]);
         if (e != cudaSuccess) {
             fail(ctx, DECAES_ECUDA, std::string("cudaMalloc: ") + cudaGetErrorString(e));
             return bail(DECAES_ECUDA);
