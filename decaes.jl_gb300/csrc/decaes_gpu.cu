@@ -643,9 +643,28 @@ int launch_shape(decaes_ctx *ctx, Kern kern, long stride, int *wpb, int *grid, s
     return fail(ctx, DECAES_EINVAL, "voxel kernel cannot be resident with this workspace size");
 }
 
+// The global scratch of a launch, `stride` doubles per warp: for fewer warps (no
+// fewer than half) when the budget, less `reserve` bytes, or the device does not
+// hold it for all of them.  The warps share a queue, so results stay the same.
+// More resident warps than the memory holds would otherwise refuse a call for
+// the sake of its speed.
+int scratch_buf(decaes_ctx *ctx, long stride, int *grid, int *wpb, size_t reserve, void **out) {
+    const size_t per_warp = sizeof(double) * (size_t)stride;
+    const long all = (long)*grid * *wpb;
+    const long room = (long)(dh::pool_scratch_room(*ctx, per_warp * all, reserve, dev_free) / per_warp);
+    if (!dh::shrink_launch(room, grid, wpb)) return buf(ctx, dh::kScratchBuf, per_warp * all, out);  // refused
+    int rc = DECAES_OK;
+    for (long q = 4; q >= 2; --q) {
+        if (!dh::shrink_launch(q * all / 4, grid, wpb)) break;
+        rc = buf(ctx, dh::kScratchBuf, per_warp * *grid * *wpb, out);
+        if (rc != DECAES_ECUDA) break;
+    }
+    return rc;
+}
+
 // Core: everything on device pointers; host-buffer entry points wrap it with copies.
 int run_t2map(decaes_ctx *ctx, const decaes_t2map_opts &o, const decaes_t2part_opts *po, const void *d_image,
-              int dtype, const void *d_b1, OutMap &out, cudaStream_t st, int *launches) {
+              int dtype, const void *d_b1, OutMap &out, cudaStream_t st, int *launches, size_t reserve = 0) {
     const long V = (long)o.MatrixSize[0] * o.MatrixSize[1] * o.MatrixSize[2];
     const int n = o.nT2;
     int nl = 0;
@@ -696,8 +715,16 @@ int run_t2map(decaes_ctx *ctx, const decaes_t2map_opts &o, const decaes_t2part_o
                          : (tc ? dk::k_voxels_mixed_tc : (is_mixed(o) ? dk::k_voxels_mixed : dk::k_voxels_plain));
     int wpb = launch_wpb(ctx, o, kern, wsm);
     if (int rc = launch_shape(ctx, kern, wsm, &wpb, &grid, &smem, tuned_bps(ctx, o))) return rc;
-    void *scr;
-    if (int rc = buf(ctx, "scratch", sizeof(double) * (size_t)P.scr_stride * grid * wpb, &scr)) return rc;
+    // tensor-core products of a chunk of the voxel list (bounded buffer)
+    const long ldF = 2L * dk::tc_ntiles(o.nRefAngles, n) * dk::kTcTileN;
+    const long C = std::max<long>(dk::kTcTileM, std::min<long>(kTcChunk, V));
+    void *F = nullptr, *Fexp = nullptr, *scr;
+    if (tc) {
+        if (int rc = buf(ctx, "tc_products", sizeof(float) * (size_t)C * ldF, &F)) return rc;
+        if (int rc = buf(ctx, "tc_exponents", sizeof(int) * (size_t)C, &Fexp)) return rc;
+    }
+    if (int rc = scratch_buf(ctx, P.scr_stride, &grid, &wpb, reserve, &scr)) return rc;
+    smem = (size_t)wpb * wsm * sizeof(double);
     P.scratch = (double *)scr;
     ctx->tc_chunks = 0;
     if (tc) {
@@ -706,11 +733,6 @@ int run_t2map(decaes_ctx *ctx, const decaes_t2map_opts &o, const decaes_t2part_o
         // chunk's voxel solve.  The host does not know the list's length, so
         // chunks past it launch and return at once.
         const int mpad = dk::tc_mpad(o.nTE), ntiles = dk::tc_ntiles(o.nRefAngles, n);
-        const long ldF = 2L * ntiles * dk::kTcTileN;
-        const long C = std::max<long>(dk::kTcTileM, std::min<long>(kTcChunk, V));
-        void *F, *Fexp;
-        if (int rc = buf(ctx, "tc_products", sizeof(float) * (size_t)C * ldF, &F)) return rc;
-        if (int rc = buf(ctx, "tc_exponents", sizeof(int) * (size_t)C, &Fexp)) return rc;
         dk::TcParams T{};
         T.image = d_image; T.f32 = dtype == DECAES_F32; T.V = V; T.m = o.nTE; T.mpad = mpad;
         T.vidx = (const int *)vidx; T.nvox = d_nvox; T.Bsl = B->Bsl; T.ntiles = ntiles;
@@ -938,8 +960,6 @@ static int t2map_host(decaes_ctx *ctx, const decaes_t2map_opts *mo, const decaes
     CK(cudaMemcpyAsync(d_img, image, img_bytes, cudaMemcpyHostToDevice, st));
     if (b1map) CK(cudaMemcpyAsync(d_b1, b1map, esize(dtype) * (size_t)V, cudaMemcpyHostToDevice, st));
     CK(cudaEventRecord(ctx->ev[1], st));
-    if (int rc = run_t2map(ctx, o, pout ? po : nullptr, d_img, dtype, d_b1, om, st, &launches)) return rc;
-    CK(cudaEventRecord(ctx->ev[4], st));
     const size_t n = o.nT2, m = o.nTE;
     struct { const double *s; void *d; size_t len; } cp[] = {
         {om.dist, mout->dist, V * n}, {om.gdn, mout->gdn, (size_t)V}, {om.ggm, mout->ggm, (size_t)V},
@@ -949,6 +969,13 @@ static int t2map_host(decaes_ctx *ctx, const decaes_t2map_opts *mo, const decaes
     };
     struct { const double *s; void *d; } pc[] = {{om.sfr, pout ? pout->sfr : nullptr}, {om.sgm, pout ? pout->sgm : nullptr},
                                                  {om.mfr, pout ? pout->mfr : nullptr}, {om.mgm, pout ? pout->mgm : nullptr}};
+    size_t reserve = 0;  // a float call's largest output, to be narrowed alone at worst
+    if (dtype == DECAES_F32) {
+        for (auto &c : cp) if (c.s && c.d) reserve = std::max(reserve, sizeof(float) * c.len);
+        for (auto &c : pc) if (c.s && c.d) reserve = std::max(reserve, sizeof(float) * (size_t)V);
+    }
+    if (int rc = run_t2map(ctx, o, pout ? po : nullptr, d_img, dtype, d_b1, om, st, &launches, reserve)) return rc;
+    CK(cudaEventRecord(ctx->ev[4], st));
     // a float call's requested outputs narrowed in one launch, packed, and copied
     // without a wait between them; one by one when there is no room for all
     std::vector<std::tuple<const double *, void *, size_t>> want;
@@ -1294,6 +1321,29 @@ int batch_plan(decaes_ctx *ctx, const decaes_volume *vols, int nvol, cudaStream_
     return DECAES_OK;
 }
 
+// The classes' launches cut to `room` bytes of scratch (as scratch_buf does for
+// one launch) and the scratch had by get(bytes), an error code: less of it while
+// the device refuses.  *scr_doubles: what all warps of all classes need, then
+// what they got.
+template <class Get>
+int batch_scratch(decaes_ctx *ctx, std::vector<BatchClass> &classes, size_t room, long *scr_doubles, Get get) {
+    const size_t all = sizeof(double) * (size_t)*scr_doubles;
+    int rc = DECAES_OK;
+    for (size_t q = 4; q >= 2; --q) {
+        *scr_doubles = 0;
+        for (BatchClass &c : classes) {
+            const size_t fit = std::min(room, q == 4 ? all : all / 4 * q) / (sizeof(double) * (size_t)c.scr_stride);
+            if (!dh::shrink_launch((long)fit, &c.grid, &c.wpb))
+                return rc ? rc : fail(ctx, DECAES_ENOMEM, "the batch's scratch (" + std::to_string(all) + " bytes) exceeds the HBM budget");
+            c.smem = (size_t)c.wpb * c.smem_stride * sizeof(double);
+            *scr_doubles = std::max(*scr_doubles, c.scr_stride * c.grid * c.wpb);
+        }
+        rc = get(sizeof(double) * (size_t)std::max<long>(*scr_doubles, 1));
+        if (rc != DECAES_ECUDA) break;
+    }
+    return rc;
+}
+
 size_t batch_bytes(const BatchPrep &bp, size_t *b_out, size_t *b_vidx, size_t *b_w, size_t *b_par, size_t *b_scr) {
     *b_out = sizeof(double) * std::max<size_t>(bp.n_out, 1);
     *b_vidx = sizeof(int) * std::max<size_t>(bp.n_vidx, 1);
@@ -1412,7 +1462,9 @@ extern "C" int decaes_t2map_t2part_batch(decaes_ctx *ctx, const decaes_volume *v
     if (int rc = buf(ctx, "batch_vidx", b_vidx, &vidx)) return rc;
     if (int rc = buf(ctx, "batch_weights", b_w, &w)) return rc;
     if (int rc = buf(ctx, "batch_params", b_par, &par)) return rc;
-    if (int rc = buf(ctx, "scratch", b_scr, &scr)) return rc;
+    if (int rc = batch_scratch(ctx, bp.classes, dh::pool_scratch_room(*ctx, b_scr, 0, dev_free), &bp.scr_doubles,
+                               [&](size_t bytes) { return buf(ctx, dh::kScratchBuf, bytes, &scr); }))
+        return rc;
     CK(cudaStreamSynchronize(st));  // the named buffers may still be in use by earlier work on this stream
     if (int rc = batch_bind(ctx, bp, outs, vidx, w, par, scr)) return rc;
     if (int rc = batch_enqueue(ctx, bp, st, &launches)) return rc;
@@ -1444,21 +1496,23 @@ extern "C" decaes_batch *decaes_batch_create(decaes_ctx *ctx, const decaes_volum
     if (int rc = batch_plan(ctx, vols, nvol, ctx->stream, b->bp, &launches)) return bail(rc);
     size_t sz[5];
     const size_t total = batch_bytes(b->bp, &sz[0], &sz[1], &sz[2], &sz[3], &sz[4]);
-    if (!fits(ctx, total)) {
-        fail(ctx, DECAES_ENOMEM, "the batch's working buffers (" + std::to_string(total) + " bytes) exceed the HBM budget");
-        return bail(DECAES_ENOMEM);
-    }
+    fits(ctx, total);  // (frees what the context holds beyond need)
+    const size_t rest = total - sz[4], room = ctx->budget > ctx->used + rest ? ctx->budget - ctx->used - rest : 0;
     void *p[5];
-    for (int i = 0; i < 5; ++i) {
-        cudaError_t e = dev_alloc(ctx, &p[i], sz[i]);
-        if (e != cudaSuccess) {
-            fail(ctx, DECAES_ECUDA, std::string("cudaMalloc: ") + cudaGetErrorString(e));
-            return bail(DECAES_ECUDA);
-        }
+    auto take = [&](int i, size_t bytes) -> int {
+        if (!fits(ctx, bytes))
+            return fail(ctx, DECAES_ENOMEM, "the batch's working buffers (" + std::to_string(total) + " bytes) exceed the HBM budget");
+        cudaError_t e = dev_alloc(ctx, &p[i], bytes);
+        if (e != cudaSuccess) return fail(ctx, DECAES_ECUDA, std::string("cudaMalloc: ") + cudaGetErrorString(e));
         b->owned.push_back(p[i]);
-        b->owned_bytes += sz[i];
-        ctx->used += sz[i];
-    }
+        b->owned_bytes += bytes;
+        ctx->used += bytes;
+        return DECAES_OK;
+    };
+    for (int i = 0; i < 4; ++i)
+        if (int rc = take(i, sz[i])) return bail(rc);
+    if (int rc = batch_scratch(ctx, b->bp.classes, room, &b->bp.scr_doubles, [&](size_t bytes) { return take(4, bytes); }))
+        return bail(rc);
     if (cudaStreamSynchronize(ctx->stream) != cudaSuccess) { fail(ctx, DECAES_ECUDA, "basis preparation failed"); return bail(0); }
     if (int rc = batch_bind(ctx, b->bp, p[0], p[1], p[2], p[3], p[4])) return bail(rc);
     if (cudaStreamCreateWithFlags(&b->cap, cudaStreamNonBlocking) != cudaSuccess) {
@@ -1888,13 +1942,15 @@ std::vector<Chunk> srv_launch_tick(decaes_server *S) {
         ok = launch_shape(ctx, k.kern, k.smem_stride, &k.wpb, &k.grid, &k.smem, tuned_bps(ctx, ch[k.first].r->mo)) == DECAES_OK;
         scr_doubles = std::max(scr_doubles, k.scr_stride * k.grid * k.wpb);
     }
-    const size_t need = sizeof(double) * (size_t)scr_doubles;
-    if (ok && need > S->scratch_bytes) {
+    ok = ok && batch_scratch(ctx, classes, SIZE_MAX, &scr_doubles, [&](size_t need) -> int {
+        if (need <= S->scratch_bytes) return DECAES_OK;
         if (S->d_scratch) cudaFreeAsync(S->d_scratch, S->comp);
         S->d_scratch = nullptr;
-        ok = cudaMallocAsync((void **)&S->d_scratch, need, S->comp) == cudaSuccess;
-        S->scratch_bytes = ok ? need : 0;
-    }
+        const bool had = cudaMallocAsync((void **)&S->d_scratch, need, S->comp) == cudaSuccess;
+        if (!had) { cudaGetLastError(); S->d_scratch = nullptr; }
+        S->scratch_bytes = had ? need : 0;
+        return had ? DECAES_OK : DECAES_ECUDA;
+    }) == DECAES_OK;
     cudaStream_t st = S->comp;
     const int ncls = (int)classes.size();
     int *counts = S->d_cnt, *offsets = S->d_cnt + nq, *counters = offsets + nq + ncls;

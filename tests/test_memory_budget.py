@@ -1,6 +1,8 @@
 """Device memory under a budget, or on a device that refuses: what the
-narrowing buffer of host float calls holds is given up before anything is
-refused for lack of it."""
+narrowing buffer of host float calls and the warps' scratch hold is given up
+before anything is refused for lack of it, and a launch whose scratch does not
+fit runs with fewer warps, to the same outputs."""
+import ctypes as C
 import os
 import shutil
 import subprocess
@@ -11,6 +13,7 @@ import pytest
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
 POOL = r"""
+#include <algorithm>
 #include <cassert>
 #include <cstdlib>
 #include "devpool.h"
@@ -48,6 +51,32 @@ int main() {
         assert(dh::pool_get(c, dh::kNarrowBuf, 31, alloc, free_, &p) == dh::kPoolOverBudget && c.used == 70);
         assert(dh::pool_get(c, "image", 101, alloc, free_, &p) == dh::kPoolOverBudget && c.used == 0 && held == 0);
     }
+    {   // the scratch: room for it beside a reserve, dropped for other buffers, never for the narrowing one
+        room = 1000; held = 0;
+        Ctx c{100};
+        assert(dh::pool_get(c, "outputs", 30, alloc, free_, &p) == dh::kPoolOk);
+        assert(dh::pool_scratch_room(c, 60, 10, free_) == 60);
+        assert(dh::pool_get(c, dh::kScratchBuf, 60, alloc, free_, &p) == dh::kPoolOk);
+        assert(dh::pool_get(c, dh::kNarrowBuf, 10, alloc, free_, &p) == dh::kPoolOk && c.used == 100);
+        assert(dh::pool_scratch_room(c, 60, 10, free_) == 60 && c.used == 100);      // fits: nothing freed
+        assert(dh::pool_scratch_room(c, 61, 10, free_) == 60 && c.used == 90);       // without the narrowing buffer
+        assert(dh::pool_scratch_room(c, 61, 20, free_) == 50 && c.used == 30);       // and the scratch is too large
+        assert(dh::pool_get(c, dh::kScratchBuf, 50, alloc, free_, &p) == dh::kPoolOk);
+        assert(dh::pool_get(c, dh::kNarrowBuf, 21, alloc, free_, &p) == dh::kPoolOverBudget && c.used == 80);
+        assert(dh::pool_get(c, "image", 21, alloc, free_, &p) == dh::kPoolOk && c.used == 51);
+        assert(dh::pool_scratch_room(c, 60, 200, free_) == 0);
+    }
+    for (int g0 = 1; g0 < 40; ++g0)                  // a cut launch fits, keeps half of the warps, or is refused
+        for (int w0 = 1; w0 <= 16; ++w0)
+            for (long fit = 0; fit <= 2L * g0 * w0; ++fit) {
+                int g = g0, w = w0;
+                const bool ok = dh::shrink_launch(fit, &g, &w);
+                assert(ok == (2 * fit >= (long)g0 * w0));
+                if (!ok) { assert(g == g0 && w == w0); continue; }
+                assert(g >= 1 && w >= 1 && g <= g0 && w <= w0 && ((long)g * w <= fit || fit >= (long)g0 * w0));
+                assert(fit < (long)g0 * w0 || (g == g0 && w == w0));
+                assert(3L * g * w >= std::min(fit, (long)g0 * w0));
+            }
     return 0;
 }
 """
@@ -111,4 +140,77 @@ def test_double_call_after_float_call_within_the_budget(D, ctx):
     _same(_call(D, tight, f32, X, m, n), want32)
     _same(_call(D, tight, img, X, m, n), want64)
     _same(_call(D, tight, f32, X, m, n), want32)  # now without room for all of them together
+    tight.close()
+
+
+def _scratch_bytes(m, n, K):
+    """Global scratch of one warp: basis, surrogate samples, caches, singular values, stored solutions, FP32 basis."""
+    return 8 * (m * n + 3 * K + 19 * 128 + min(m, n) + 16 + 64 * (n + 1) + (m * n + 1) // 2)
+
+
+# Budgets for the scratch of as many warps per SM as single-warp blocks with the
+# whole workspace in shared memory hold (12 mixed, 3 plain), and 8 MB for
+# the rest: fewer than the launches' own shapes (15, 4) take.
+@pytest.mark.gpu
+@pytest.mark.parametrize("m,n,precision,warps", [(48, 40, "mixed", 12), (56, 60, "fp64", 3)])
+def test_fewer_warps_where_the_scratch_does_not_fit(D, ctx, m, n, precision, warps):
+    import torch
+    X, K = (5, 4, 3), 8
+    img = D.mock_image(D.MockImageOptions(MatrixSize=X, nTE=m), seed=4)
+    mo = D.T2mapOptions(MatrixSize=X, nTE=m, TE=10e-3, nT2=n, T2Range=(10e-3, 2.0), Reg="lcurve", nRefAngles=K,
+                        precision=precision)
+    po = D.T2partOptions.from_t2map(mo, SPWin=(10e-3, 25e-3), MPWin=(25e-3, 200e-3))
+
+    def host(c, dt):
+        maps, dist, parts = D.T2mapSEcorr_T2partSEcorr(np.asfortranarray(img, dtype=dt), mo, po, ctx=c)
+        return dict(maps, dist=dist, **parts)
+
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    tight = D.Context(0, hbm_budget_bytes=warps * sms * _scratch_bytes(m, n, K) + (8 << 20))
+    for dt in (np.float32, np.float64):
+        _same(host(tight, dt), host(ctx, dt))
+    tight.close()
+    with pytest.raises(RuntimeError, match="ENOMEM"):  # a quarter of the warps is still refused
+        host(D.Context(0, hbm_budget_bytes=warps * sms * _scratch_bytes(m, n, K) // 4), np.float64)
+
+
+# the same for batches (one-shot, prepared), two classes
+@pytest.mark.gpu
+def test_batches_with_fewer_warps_where_the_scratch_does_not_fit(D, ctx):
+    import torch
+    from decaes_gb300 import _lib
+    L = D.load()
+    X, K, V = (4, 3, 2), 8, 24
+    vols, outs = [], []
+    for i, (m, n) in enumerate([(48, 40), (64, 60)]):
+        img = D.mock_image(D.MockImageOptions(MatrixSize=X, nTE=m), seed=6 + i)
+        mo = D.T2mapOptions(MatrixSize=X, nTE=m, TE=10e-3, nT2=n, T2Range=(10e-3, 2.0), Reg="chi2", Chi2Factor=1.02,
+                            nRefAngles=K, precision="mixed")
+        _, dist = D.T2mapSEcorr(img, mo, ctx=ctx)
+        d_img = torch.from_numpy(img.reshape(-1, order="F").copy()).cuda()
+        out = {k: torch.full((V * (n if k == "dist" else 1),), 7.0, dtype=torch.float64, device="cuda")
+               for k in ("dist", "gdn", "ggm", "gva", "fnr", "snr", "alpha")}
+        vols.append(_lib.VolumeC(mopts=mo.to_c(), has_t2part=0, dtype=_lib.F64, d_image=d_img.data_ptr(), d_b1map=None,
+                                 d_mout=_lib.T2mapOutC(**{k: t.data_ptr() for k, t in out.items()})))
+        outs.append((d_img, out, dist.reshape(-1, order="F")))
+    arr = (_lib.VolumeC * len(vols))(*vols)
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    # 12 warps per SM of the smaller volume, 5 of the larger; 15 and 7 are launched
+    need = sms * max(12 * _scratch_bytes(48, 40, K), 5 * _scratch_bytes(64, 60, K))
+    tight = D.Context(0, hbm_budget_bytes=need + (16 << 20))
+
+    def check():
+        torch.cuda.synchronize()
+        for _, out, want in outs:
+            np.testing.assert_array_equal(out["dist"].cpu().numpy(), want)
+            out["dist"].fill_(7.0)
+
+    torch.cuda.synchronize()
+    tight.check(L.decaes_t2map_t2part_batch(tight.h, arr, len(vols), None))
+    check()
+    b = L.decaes_batch_create(tight.h, arr, len(vols))
+    assert b, L.decaes_last_error(tight.h).decode()
+    assert L.decaes_batch_run(b, None) == 0
+    check()
+    L.decaes_batch_destroy(b)
     tight.close()
