@@ -387,6 +387,16 @@ int buf(decaes_ctx *ctx, const std::string &name, size_t bytes, void **out) {
     }
 }
 
+// Milliseconds between two events; 0 when either was never recorded (a context
+// that has run no single-volume call), without leaving that error pending for
+// the next call's checks.
+float elapsed_ms(cudaEvent_t a, cudaEvent_t b) {
+    float t = 0.f;
+    if (cudaEventElapsedTime(&t, a, b) == cudaSuccess) return t;
+    cudaGetLastError();
+    return 0.f;
+}
+
 size_t esize(int dtype) { return dtype == DECAES_F32 ? 4 : 8; }
 
 // The mixed method, with the grid products from the CUDA cores or the tensor cores.
@@ -1103,18 +1113,18 @@ extern "C" int decaes_sync_stats(decaes_ctx *ctx, void *stream) {
     if (!ctx) return DECAES_EINVAL;
     cudaStream_t st = stream ? (cudaStream_t)stream : ctx->stream;
     CK(cudaStreamSynchronize(st));
-    void *cnt;
-    if (int rc = buf(ctx, "counters", 64, &cnt)) return rc;
-    int hn;
-    unsigned long long hs[2];
-    CK(cudaMemcpy(&hn, cnt, sizeof(int), cudaMemcpyDeviceToHost));
-    CK(cudaMemcpy(hs, (char *)cnt + 16, sizeof hs, cudaMemcpyDeviceToHost));
-    float t;
+    const void *cnt = ctx->bufs["counters"].p;
+    int hn = 0;
+    unsigned long long hs[2] = {0, 0};
+    if (cnt) {
+        CK(cudaMemcpy(&hn, cnt, sizeof(int), cudaMemcpyDeviceToHost));
+        CK(cudaMemcpy(hs, (const char *)cnt + 16, sizeof hs, cudaMemcpyDeviceToHost));
+    }
     ctx->stats.voxels_processed = hn;
     ctx->stats.nnls_cap_hits = (int64_t)hs[0];
     ctx->stats.search_limit_hits = (int64_t)hs[1];
-    cudaEventElapsedTime(&t, ctx->ev[0], ctx->ev[5]); ctx->stats.ms_total = t;
-    cudaEventElapsedTime(&t, ctx->ev[2], ctx->ev[3]); ctx->stats.ms_solve = t;
+    ctx->stats.ms_total = elapsed_ms(ctx->ev[0], ctx->ev[5]);
+    ctx->stats.ms_solve = elapsed_ms(ctx->ev[2], ctx->ev[3]);
     fill_tc_stats(ctx, cnt);
     return DECAES_OK;
 }
