@@ -11,6 +11,7 @@
 #include <chrono>
 #include <cmath>
 #include <condition_variable>
+#include <cstddef>
 #include <cstdio>
 #include <cstring>
 #include <deque>
@@ -333,8 +334,9 @@ struct decaes_ctx {
     size_t smem_optin = 0;
     std::map<TuneKey, Tune> tune;
     std::map<std::pair<const void *, long>, int> wpb;  // most_warps_wpb per kernel and workspace
-    int force_wpb = 0;  // autotuner trials
+    int force_wpb = 0;  // autotuner trials (-1: the default shape)
     int force_bps = 0;
+    int last_wpb = 0, last_bps = 0;  // the last single-volume launch: warps per block, blocks per SM
     int tc_chunks = 0;                 // tensor-core product launches of the last call
     cudaEvent_t tc_ev[2 * kTcEvents];  // their start/end events (the first kTcEvents)
     std::mutex mu;
@@ -561,7 +563,7 @@ int make_params(decaes_ctx *ctx, const decaes_t2map_opts &o, const dh::T2partPla
 // Warps per block for a launch of these options: forced, else autotuned,
 // else 0 (no preference).
 int tuned_wpb_or0(decaes_ctx *ctx, const decaes_t2map_opts &o) {
-    if (ctx->force_wpb) return ctx->force_wpb;
+    if (ctx->force_wpb) return std::max(ctx->force_wpb, 0);
     const bool fixed = !std::isnan(o.SetFlipAngle);
     TuneKey k{o.nTE, o.nT2, fixed ? 1 : o.nRefAngles, o.Reg, is_mixed(o), o.RefConAngle == 180.0,
               o.legacy != 0};
@@ -571,7 +573,7 @@ int tuned_wpb_or0(decaes_ctx *ctx, const decaes_t2map_opts &o) {
 // Resident blocks per SM for a launch of these options: forced, else
 // autotuned, else 0 (as many as fit).
 int tuned_bps(decaes_ctx *ctx, const decaes_t2map_opts &o) {
-    if (ctx->force_bps) return ctx->force_bps;
+    if (ctx->force_wpb) return ctx->force_bps;
     const bool fixed = !std::isnan(o.SetFlipAngle);
     TuneKey k{o.nTE, o.nT2, fixed ? 1 : o.nRefAngles, o.Reg, is_mixed(o), o.RefConAngle == 180.0, o.legacy != 0};
     auto it = ctx->tune.find(k);
@@ -735,6 +737,8 @@ int run_t2map(decaes_ctx *ctx, const decaes_t2map_opts &o, const decaes_t2part_o
     }
     if (int rc = scratch_buf(ctx, P.scr_stride, &grid, &wpb, reserve, &scr)) return rc;
     smem = (size_t)wpb * wsm * sizeof(double);
+    ctx->last_wpb = wpb;
+    ctx->last_bps = (grid + ctx->sms - 1) / ctx->sms;
     P.scratch = (double *)scr;
     ctx->tc_chunks = 0;
     if (tc) {
@@ -1573,6 +1577,10 @@ extern "C" void decaes_batch_destroy(decaes_batch *b) {
     delete b;
 }
 
+// (the two kept_ fields lie where the struct's first form had padding)
+static_assert(offsetof(decaes_tuning, us_per_voxel) == 8 && offsetof(decaes_tuning, blocks_per_sm) == 16 &&
+                  sizeof(decaes_tuning) == 24, "decaes_tuning keeps its layout");
+
 extern "C" int decaes_autotune(decaes_ctx *ctx, const decaes_t2map_opts *opts, decaes_tuning *out) {
     if (int rc = check_both(ctx, opts, nullptr, DECAES_F32)) return rc;
     std::lock_guard<std::mutex> lk(ctx->mu);
@@ -1606,8 +1614,9 @@ extern "C" int decaes_autotune(decaes_ctx *ctx, const decaes_t2map_opts *opts, d
     // two fewer (fewer warps sharing an SM's FP64 pipes, L1 and L2 share); then
     // the default shape of an untuned call, which stays when it is the fastest.
     const int cand[3] = {1, 2, 4};
-    int best_w = 1, best_b = 0;
+    int best_w = 1, best_b = 0, kept_w = 0, kept_b = 0;
     double best_ms = 1e30;
+    struct Unforce { decaes_ctx *c; ~Unforce() { c->force_wpb = c->force_bps = 0; } } unforce{ctx};
     auto trial = [&](int w, int b, float *ms) -> int {
         ctx->force_wpb = w;
         ctx->force_bps = b;
@@ -1623,43 +1632,43 @@ extern "C" int decaes_autotune(decaes_ctx *ctx, const decaes_t2map_opts *opts, d
         *ms = best;
         return DECAES_OK;
     };
+    auto better = [&](float t, int w, int b) {
+        if (t >= best_ms) return;
+        best_ms = t; best_w = w; best_b = b;
+        kept_w = ctx->last_wpb; kept_b = ctx->last_bps;
+    };
     for (int w : cand) {
         float t = 0;
-        int rc = trial(w, 0, &t);
-        if (rc) { ctx->force_wpb = ctx->force_bps = 0; return rc; }
-        if (t < best_ms) { best_ms = t; best_w = w; best_b = 0; }
+        if (int rc = trial(w, 0, &t)) return rc;
         // blocks per SM of the full grid of this block size
         Basis *B = nullptr;
         dk::Params P;
         long wsm = 0;
         int wpb = w, grid = 0;
         size_t smem = 0;
-        if ((rc = get_basis(ctx, o, &B)) || (rc = make_params(ctx, o, nullptr, nullptr, B, d_img, DECAES_F32, nullptr, om, P, &wsm))) {
-            ctx->force_wpb = ctx->force_bps = 0;
-            return rc;
-        }
+        if (int rc = get_basis(ctx, o, &B)) return rc;
+        if (int rc = make_params(ctx, o, nullptr, nullptr, B, d_img, DECAES_F32, nullptr, om, P, &wsm)) return rc;
         auto kern = o.legacy ? dk::k_voxels_legacy : (is_mixed(o) ? dk::k_voxels_mixed : dk::k_voxels_plain);
-        if ((rc = launch_shape(ctx, kern, wsm, &wpb, &grid, &smem))) { ctx->force_wpb = ctx->force_bps = 0; return rc; }
-        if (wpb != w) continue;  // this block size does not fit
+        if (int rc = launch_shape(ctx, kern, wsm, &wpb, &grid, &smem)) return rc;
+        if (wpb != w) continue;  // this block size does not fit: the trial ran a smaller one
+        better(t, w, 0);
         const int full = grid / ctx->sms;
         for (int b = full - 1; b >= std::max(1, full - 2); --b) {
-            if ((rc = trial(w, b, &t))) { ctx->force_wpb = ctx->force_bps = 0; return rc; }
-            if (t < best_ms) { best_ms = t; best_w = w; best_b = b; }
+            if (int rc = trial(w, b, &t)) return rc;
+            better(t, w, b);
         }
     }
-    ctx->force_wpb = ctx->force_bps = 0;
-    const bool fixed = !std::isnan(o.SetFlipAngle);
-    TuneKey k{o.nTE, o.nT2, fixed ? 1 : o.nRefAngles, o.Reg, is_mixed(o), o.RefConAngle == 180.0,
-              o.legacy != 0};
-    ctx->tune.erase(k);
     float t_default = 0;
-    if (int rc = trial(0, 0, &t_default)) return rc;
-    Tune t;
-    t.wpb = t_default <= best_ms ? 0 : best_w;
-    t.bps = t_default <= best_ms ? 0 : best_b;
-    t.us_per_voxel = std::min<double>(t_default, best_ms) * 1e3 / (double)V;
-    ctx->tune[k] = t;
-    if (out) { out->warps_per_block = best_w; out->us_per_voxel = t.us_per_voxel; out->blocks_per_sm = best_b; }
+    if (int rc = trial(-1, 0, &t_default)) return rc;
+    Tune t{best_w, best_b, best_ms * 1e3 / (double)V};
+    if (t_default <= best_ms) {
+        t = Tune{0, 0, t_default * 1e3 / (double)V};
+        kept_w = ctx->last_wpb; kept_b = ctx->last_bps;
+    }
+    // an earlier tuning of this shape stays until here, where nothing can fail
+    const bool fixed = !std::isnan(o.SetFlipAngle);
+    ctx->tune[TuneKey{o.nTE, o.nT2, fixed ? 1 : o.nRefAngles, o.Reg, is_mixed(o), o.RefConAngle == 180.0, o.legacy != 0}] = t;
+    if (out) *out = decaes_tuning{best_w, kept_w, t.us_per_voxel, best_b, kept_b};
     return DECAES_OK;
 }
 

@@ -216,15 +216,21 @@ void decaes_batch_destroy(decaes_batch *batch);
  * and method for a set of launch shapes -- 1, 2 and 4 warps (voxels in
  * flight) per block, each with as many resident blocks per SM as fit and with
  * one and two fewer -- and for the shape an untuned call takes (the block size
- * that keeps the most warps resident), and keeps the fastest for that (nTE,
- * nT2, nRefAngles, Reg, precision, control angle) in the context.  It reports
- * the fastest of the former and the cost of the shape kept.  Later calls,
- * batches and server ticks on the context use the kept shape; batches also use
- * the measured cost to order their queue. */
+ * that keeps the most warps resident), and keeps the fastest of them all for
+ * that (nTE, nT2, nRefAngles, Reg, precision, control angle) in the context.
+ * warps_per_block and blocks_per_sm report the fastest of the block sizes 1, 2
+ * and 4; kept_warps_per_block and kept_blocks_per_sm the shape kept, which is
+ * that one or the untuned one, as launched by the trial; us_per_voxel is the
+ * kept shape's.  Later calls, batches and server ticks on the context use the
+ * kept shape; batches also use the measured cost to order their queue.  A call
+ * that fails keeps what an earlier one tuned.  (The struct has the size and the
+ * offsets it had without the kept_ fields.) */
 typedef struct {
     int32_t warps_per_block;
+    int32_t kept_warps_per_block;
     double us_per_voxel;       /* device time per above-threshold voxel, whole GPU */
     int32_t blocks_per_sm;     /* resident blocks per SM (0: as many as fit) */
+    int32_t kept_blocks_per_sm;
 } decaes_tuning;
 int decaes_autotune(decaes_ctx *ctx, const decaes_t2map_opts *opts, decaes_tuning *out);
 
