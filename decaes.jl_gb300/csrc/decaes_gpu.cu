@@ -585,6 +585,8 @@ int tuned_bps(decaes_ctx *ctx, const decaes_t2map_opts &o) {
 // of its own besides its warps' workspaces, so one large block can hold a warp
 // or two more than single-warp blocks do (mixed method at 40 T2 times 15
 // instead of 13, at 60 with GCV 7 instead of 6).  Ties go to the smaller block.
+// Such a block keeps its SM's shared memory until its last warp is done, so the
+// next launch's blocks, of another stream too, wait for whole blocks.
 template <class Kern>
 int most_warps_wpb(decaes_ctx *ctx, Kern kern, long stride) {
     const auto key = std::make_pair((const void *)kern, stride);
@@ -619,9 +621,14 @@ int launch_wpb(decaes_ctx *ctx, const decaes_t2map_opts &o, Kern kern, long stri
 // that half the solves would leave shared memory).  FP64 method, 64x64x1 voxels:
 // 56 echoes x 60 T2 times (3 -> 4 warps) chi2 43.3 -> 36.1 ms, GCV 94.4 -> 77.4;
 // 48 x 48 (5 -> 6) L-curve 57.8 -> 49.0; 48 x 40 (7 -> 8) L-curve, 120x120x1,
-// 115.0 -> 113.0 ms.
+// 115.0 -> 113.0 ms.  The spilled calls' out-of-line copies cost the kernel
+// registers around every solve (spill stores / loads 108 / 180 -> 1,060 / 1,556
+// bytes): ~1% of a call that spills no row, 8x8x2 chi2 5.49 -> 5.54 ms.  Shapes
+// that hold eight warps already (32 x 40 and smaller) keep their matrix whole: a
+// ninth, in several blocks, which registers would allow, has not been measured.
+// Tuned shapes, batches and served ticks keep it whole as well.
 void spill_rows(decaes_ctx *ctx, int m, int n, dk::Params &P, long *wsm) {
-    constexpr int kMaxWarps = 8;  // of the plain kernel's block
+    constexpr int kMaxWarps = 8;  // (see above)
     const long avail = (long)(ctx->smem_optin / sizeof(double));
     const long w = avail / *wsm + 1;
     if (w < 2 || w > kMaxWarps) return;

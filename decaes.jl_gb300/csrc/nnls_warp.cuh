@@ -144,7 +144,8 @@ extern __shared__ __align__(16) double dk_smem[];
 // window check, a longer latency and two address instructions instead of one).
 // Indexing dk_smem itself keeps them 32-bit shared-memory accesses:
 // 240x240x1 x 48 echoes, L-curve: mixed 72.1 -> 66.3 ms; 120x120x1 FP64 method
-// 136.7 -> 131.2 ms, and no register spills in either kernel.
+// 136.7 -> 131.2 ms.  (Bytes of register spills, stores / loads, by that change:
+// k_voxels_plain 328 / 928 -> 68 / 160, k_voxels_mixed 0 / 0 -> 112 / 228.)
 template <class T>
 struct Sh {
     int off;
@@ -230,8 +231,8 @@ __device__ __forceinline__ void copy_async_wait() {
 // Per-warp views of the NNLS workspace (shared memory).
 struct NnlsWS {
     ShD C;    // lda x n, physical columns
-    ShD b;    // lda (right-hand side, transformed in place)
-    ShD zz;   // lda
+    ShD b;    // (m + n) | 1 whatever lda is (right-hand side, transformed in place)
+    ShD zz;   // (m + n) | 1
     ShD x;    // n, indexed by original column (0-based)
     ShD w;    // n, indexed by logical position (0-based)
     ShI idx;  // n, 1-based original column at each logical position

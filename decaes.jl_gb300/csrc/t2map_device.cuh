@@ -38,8 +38,8 @@ constexpr bool kTcProducts = DECAES_TC_PRODUCTS != 0;
 
 // Helpers with several call sites on the mixed method's hot path are kept out
 // of line in its single-method kernel (one copy in the instruction cache
-// instead of one per site: the kernel is ~0.5 MB of code and instruction
-// fetch is a visible stall); the other kernels inline them as before.
+// instead of one per site: the kernel is several hundred KB of code and
+// instruction fetch is a visible stall); the other kernels inline them as before.
 #if DECAES_METHODS == 2
 #define DK_OUTLINE __noinline__
 #else

@@ -100,8 +100,10 @@ __host__ __device__ inline long warp_smem_doubles_mixed(int m, int n, bool gcv) 
 }
 // Lanes of the FP64 method's EPG basis (one T2 column per lane, 3 * ((m + 1) / 2
 // + 1) states each).  The states use the contiguous C, b and zz regions of the
-// workspace (lda * (n + 2) doubles, free while the voxel's basis is built), which
-// hold at least one lane's states for every n >= 1 because lda >= m + n.
+// workspace (free while the voxel's basis is built): lda * n + 2 ((m + n) | 1)
+// doubles, at least lda * (n + 2) because lda <= (m + n) | 1.  One lane's states
+// always fit: lda >= m and n >= 2 (rows may lie elsewhere, lda >= max(m, n) | 1),
+// so they have 4 m doubles and need 3 m at most (m >= 4).
 __host__ __device__ inline int fp64_epg_lanes(int m, int n, int lda) {
     long l = ((long)lda * (n + 2)) / (3L * ((m + 1) / 2 + 1));
     return (int)(l < 1 ? 1 : (l > 32 ? 32 : l));

@@ -2,7 +2,6 @@
 narrowing buffer of host float calls and the warps' scratch hold is given up
 before anything is refused for lack of it, and a launch whose scratch does not
 fit runs with fewer warps, to the same outputs."""
-import ctypes as C
 import os
 import shutil
 import subprocess
